@@ -1400,6 +1400,10 @@ void autotune_impl(Ctx &c) {
     const int p2g0 = c.p2g_var, g2p0 = c.g2p_var;
     try {
         EXG_CUDA_OK(cudaMemsetAsync(&c.ctl->maxppc, 0, sizeof(int), c.stream));
+        // the touched-tile list of the sort starts empty, as in a step: the
+        // last step's count is still in the control block, and a list
+        // appended to it would run past its ntiles entries
+        EXG_CUDA_OK(cudaMemsetAsync(&c.ctl->n_touched_tiles, 0, sizeof(int), c.stream));
         do_sort(c, true);
         launch_reset_accum(c, c.bounds2, c.dtmin2);
         DISPATCH(launch_state_reduce, c, c.bounds2, c.dtmin2);

@@ -113,3 +113,30 @@ def test_tma_and_plain_node_staging_agree(name, precision, monkeypatch):
     monkeypatch.setenv("EXG_NO_TMA", "1")
     got, _ = run(s, p, 8, 0, 0)
     assert same(got, ref)
+
+
+def test_tuning_leaves_device_memory_alone():
+    """A tuning run between two steps starts its own list of touched tiles:
+    the first step of a context touches every tile, so a list appended to that
+    step's would overrun into the allocations behind it (the material table
+    among them) and change the steps that follow."""
+    dx = 1.0 / 256
+    n = (101, 48, 51)
+    size = tuple(k * dx for k in n)
+    s, p = scenes.dam_break(n=n, size=size, block=(0.4 * size[0], size[1], 0.6 * size[2]), seed=6)
+    s.autotune = 0
+    out = []
+    for tune in (False, True):
+        ctx = nt.Context(s)
+        ctx.upload(p)
+        ctx.Initialise_Internal_Forces()
+        ctx.step(1)
+        if tune:
+            ctx.autotune()
+        ctx.step(3)
+        out.append((ctx.download(), ctx.time()))
+        ctx.close()
+    (a, ta), (b, tb) = out
+    assert ta == tb
+    assert np.array_equal(a.pos, b.pos)
+    assert np.array_equal(a.rdata, b.rdata)
