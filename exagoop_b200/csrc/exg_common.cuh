@@ -119,6 +119,12 @@ struct Params {
     int ntile[3];
     long long ntiles;
     int hlo, hhi, B;    // node-block halo below/above and edge B = T+hlo+hhi
+    // P2G work items per tile, 1 << pshift: each takes T >> pshift z planes of
+    // cells and leaves a node block of B x B x Bz (see p2g_split)
+    int pshift, Bz;
+    // words between z planes of a node block: B x B, padded where that spreads
+    // the W x W columns a warp adds to over more shared-memory banks
+    int PS;
     double gravity[3];
     int external_loads;
     double slab_lo[3], slab_hi[3], extforce[3];

@@ -86,6 +86,7 @@ void launch_time_advance(Ctx &c);
 void launch_node_reset(Ctx &c);
 #define EXG_DECL_PREC(sfx)                                                      \
     void launch_state_reduce##sfx(Ctx &c, unsigned long long *bounds, unsigned long long *dtmin); \
+    bool p2g_fits##sfx(const Ctx &c, int ps);                                    \
     void launch_p2g##sfx(Ctx &c, int flags);                                     \
     void launch_nodes##sfx(Ctx &c, int mode, int flags, bool all_tiles);         \
     void launch_g2p_fused##sfx(Ctx &c, int mode);                                \
@@ -187,7 +188,7 @@ struct Ctx {
     long long *staging = nullptr;      // P2G partial node blocks (fixed point)
     double *stage = nullptr;           // one FP64 particle field: host transfers
     long long stage_cap = 0;
-    size_t staging_cap = 0;            // in tiles
+    size_t staging_cap = 0;            // in 64-bit words
     int nch = 7;
     // control block
     Ctl *ctl = nullptr;                // device

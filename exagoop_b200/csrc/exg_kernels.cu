@@ -679,33 +679,7 @@ struct Stc {
     static constexpr int LO = (ORD == 1) ? 0 : -1;
 };
 
-template <int W, class T>
-__device__ __forceinline__ T pick(const T (&a)[W], int i) {
-    if (W == 2) return i ? a[1] : a[0];
-    return i == 0 ? a[0] : (i == 1 ? a[1] : (i == 2 ? a[2] : a[W - 1]));
-}
-
-// ---------------------------------------------------------------- K2 per-cell P2G
-// P2G with one thread per cell (nearest-node bin for quadratic): the thread
-// walks its cell's particles (contiguous after the sort) in storage order
-// and accumulates their contributions to rows of one z-slice of the cell's
-// stencil in registers; only the per-cell sums go to the tile's node block
-// in shared memory, as 64-bit fixed point.  The summation order inside a
-// cell is fixed and the cross-cell sums are exact, so the result is
-// deterministic; shared-memory atomics drop by the particles-per-cell factor
-// and lanes never collide (a warp's lanes own different cells and add the
-// same stencil offset at the same time).
-template <class R>
-__device__ __forceinline__ long long to_fixed(R v, R sc);
-template <>
-__device__ __forceinline__ long long to_fixed<float>(float v, float sc) {
-    return __float2ll_rn(v * sc);
-}
-template <>
-__device__ __forceinline__ long long to_fixed<double>(double v, double sc) {
-    return __double2ll_rn(v * sc);
-}
-
+// ---------------------------------------------------------------- K2 helpers
 // A node's fixed-point sum in shared memory.
 // FP32 state (scale bound 2^55, kFxBits32): two 32-bit words; without
 // carries, lo collects the low 24 bits of each addend (at most 64 addends
@@ -737,42 +711,51 @@ __device__ __forceinline__ void fx_split64(double x, unsigned long long &lo, int
     hi = small ? (q < 0 ? -1 : 0) : (int)h;
 }
 
-// Branch-free: adding zero words changes no sum, and the straight-line
-// code keeps a warp's lanes together.
+// A node block in shared memory: n values (n a multiple of 4), FP32 the n low
+// words, then the n high words; FP64 the n 64-bit low words, then the n
+// 32-bit high words.
 template <class R>
-__device__ __forceinline__ void fx_add_r(unsigned *lo, int *hi, int idx, R v, R sc) {
-    if (sizeof(R) == 4) {
-        const long long q = to_fixed<R>(v, sc);
-        atomicAdd(&lo[idx], (unsigned)(q & 0xFFFFFFll));
-        atomicAdd(&hi[idx], (int)(q >> 24));
+__device__ __forceinline__ void fx_add_r(unsigned char *blk, int n, int idx, R v, R sc) {
+    if constexpr (sizeof(R) == 4) {
+        unsigned *lo = reinterpret_cast<unsigned *>(blk);
+        const long long q = __float2ll_rn(v * sc);
+        atomicAdd(lo + idx, (unsigned)(q & 0xFFFFFFll));
+        atomicAdd(reinterpret_cast<int *>(lo + n) + idx, (int)(q >> 24));
     } else {
         unsigned long long l;
         int h;
         fx_split64((double)v * (double)sc, l, h);
-        unsigned long long *lo64 = reinterpret_cast<unsigned long long *>(lo);
-        const unsigned long long old = atomicAdd(&lo64[idx], l);
-        atomicAdd(&hi[idx], h + ((old + l < old) ? 1 : 0));
+        unsigned long long *lo = reinterpret_cast<unsigned long long *>(blk);
+        const unsigned long long old = atomicAdd(lo + idx, l);
+        atomicAdd(reinterpret_cast<int *>(lo + n) + idx, h + ((old + l < old) ? 1 : 0));
     }
 }
-// Zeroes the tile's fixed-point block (n values) in shared memory.
+// One warp writes a node block to its staging slot and zeroes it for the
+// next item: FP32 one 64-bit integer per value; FP64 the words as they lie.
 template <class R>
-__device__ __forceinline__ void fx_zero(unsigned *lo, int *hi, int n) {
-    for (int i = threadIdx.x; i < n * fx_lo_words<R>(); i += blockDim.x) lo[i] = 0u;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) hi[i] = 0;
-}
-// Writes the tile's fixed-point block (n values) to its staging slot: FP32
-// one 64-bit integer per value; FP64 the 64-bit low words, then the 32-bit
-// high words.
-template <class R>
-__device__ __forceinline__ void fx_store(const unsigned *lo, const int *hi, int n, long long *dst) {
-    if (sizeof(R) == 4) {
-        for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = (long long)hi[i] * (1ll << 24) + (long long)lo[i];
+__device__ __forceinline__ void fx_store_zero(unsigned char *blk, int n, long long *dst) {
+    const int lane = threadIdx.x & 31;
+    if constexpr (sizeof(R) == 4) {
+        uint4 *lo = reinterpret_cast<uint4 *>(blk);
+        int4 *hi = reinterpret_cast<int4 *>(blk + 4 * (size_t)n);
+        longlong2 *d2 = reinterpret_cast<longlong2 *>(dst);
+#pragma unroll 4
+        for (int i = lane; i < n / 4; i += 32) {
+            const int4 h = hi[i];
+            const uint4 l = lo[i];
+            d2[2 * i] = make_longlong2((long long)h.x * (1ll << 24) + (long long)l.x,
+                                       (long long)h.y * (1ll << 24) + (long long)l.y);
+            d2[2 * i + 1] = make_longlong2((long long)h.z * (1ll << 24) + (long long)l.z,
+                                           (long long)h.w * (1ll << 24) + (long long)l.w);
+            hi[i] = make_int4(0, 0, 0, 0);
+            lo[i] = make_uint4(0u, 0u, 0u, 0u);
+        }
     } else {
-        const unsigned long long *lo64 = reinterpret_cast<const unsigned long long *>(lo);
-        int *dh = reinterpret_cast<int *>(dst + n);
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            dst[i] = (long long)lo64[i];
-            dh[i] = hi[i];
+        uint4 *b4 = reinterpret_cast<uint4 *>(blk), *d4 = reinterpret_cast<uint4 *>(dst);
+#pragma unroll 4
+        for (int i = lane; i < n / 4 * 3; i += 32) {  // 12 bytes a value
+            d4[i] = b4[i];
+            b4[i] = make_uint4(0u, 0u, 0u, 0u);
         }
     }
 }
@@ -823,28 +806,8 @@ struct P2GStc {
 // keeps FP32's relative precision: quadratic (1/2)(1/2 - u)^2, 3/4 - u^2,
 // (1/2)(1/2 + u)^2; cubic g^3 / 6, 2/3 + f^2 (f / 2 - 1),
 // 2/3 + g^2 (g / 2 - 1), f^3 / 6 with g = 1 - f.  The reference's truncated
-// constants round to the same floats as 1/6 and 2/3.  Per slot s (unscaled
-// derivative):
-__device__ __forceinline__ void slot_weight_f32(int ord, float f, int s, float &w, float &dw) {
-    if (ord == 3) {
-        const float t = (s == 0 || s == 2) ? 1.f - f : f, t2 = t * t;
-        if (s == 0 || s == 3) {
-            w = t2 * (t * (float)kOneBySix);
-            dw = (s == 0 ? -0.5f : 0.5f) * t2;
-        } else {
-            w = fmaf(t2, fmaf(0.5f, t, -1.f), (float)kTwoByThree);
-            dw = (s == 1 ? t : -t) * fmaf(1.5f, t, -2.f);
-        }
-    } else if (s == 1) {
-        w = fmaf(-f, f, 0.75f);
-        dw = -2.f * f;
-    } else {
-        const float t = s == 0 ? 0.5f - f : 0.5f + f;
-        w = 0.5f * (t * t);
-        dw = s == 0 ? -t : t;
-    }
-}
-
+// constants round to the same floats as 1/6 and 2/3.
+//
 // Interior weights of all W slots from the particle's offset f in its cell
 // (cubic, slot s at z = f + 1 - s) or bin (quadratic, u = offset from the
 // bin's node, slot s at u + 1 - s): the fixed pieces of the type-3 splines,
@@ -1009,503 +972,15 @@ __device__ __forceinline__ void p2g_axis_weights(const SplineTables &tab, const 
         cell_axis_weights<R, ORD>(tab, P, d, x, i, interior, a);
 }
 
-// Per-particle P2G coefficients: m, m v, the body force m g (+ the external
-// force inside the slab) and -V sigma, so that every node contribution is a
-// chain of fused multiply-adds; thermal: m cp, m cp T, m k, V q, V Q.
-template <class R, bool THERM>
-struct P2GCoef {
-    R m, mv[3], b[3], s[6];
-    R mcp, mcpT, mk, qv[3], VQ;
-};
-
-// Register accumulators of one stencil node.  FP32 keeps channel pairs in
-// float2 and adds them with the packed FP32 FMA of sm_100 (two lanes per
-// instruction): (m, p_x), (p_y, p_z), (f_x, f_y), then f_z alone.
-template <class R, bool THERM>
-struct P2GAcc {
-    R c[THERM ? CH_ALL : CH_MOM_END];
-    __device__ __forceinline__ void zero() {
-#pragma unroll
-        for (int i = 0; i < (THERM ? CH_ALL : CH_MOM_END); ++i) c[i] = R(0);
-    }
-    __device__ __forceinline__ void add(const P2GCoef<R, THERM> &q, R N, R g0, R g1, R g2) {
-        c[CH_M] = fma(q.m, N, c[CH_M]);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) c[CH_P + d] = fma(q.mv[d], N, c[CH_P + d]);
-        c[CH_F + 0] = fma(q.s[2], g2, fma(q.s[1], g1, fma(q.s[0], g0, fma(q.b[0], N, c[CH_F + 0]))));
-        c[CH_F + 1] = fma(q.s[4], g2, fma(q.s[3], g1, fma(q.s[1], g0, fma(q.b[1], N, c[CH_F + 1]))));
-        c[CH_F + 2] = fma(q.s[5], g2, fma(q.s[4], g1, fma(q.s[2], g0, fma(q.b[2], N, c[CH_F + 2]))));
-        if (THERM) add_thermal(q, N, g0, g1, g2);
-    }
-    __device__ __forceinline__ void add_thermal(const P2GCoef<R, THERM> &q, R N, R g0, R g1, R g2) {
-        if constexpr (THERM) {
-            c[CH_MC] = fma(q.mcp, N, c[CH_MC]);
-            c[CH_MCT] = fma(q.mcpT, N, c[CH_MCT]);
-            c[CH_MK] = fma(q.mk, N, c[CH_MK]);
-            c[CH_SRC] = fma(q.VQ, N, fma(q.qv[2], g2, fma(q.qv[1], g1, fma(q.qv[0], g0, c[CH_SRC]))));
-        }
-    }
-    __device__ __forceinline__ R get(int ch) const { return c[ch]; }
-};
-
-template <bool THERM>
-struct P2GAcc<float, THERM> {
-    float2 mp0, p12, f01;
-    float f2;
-    float th[4];  // m cp, m cp T, m k, source
-    __device__ __forceinline__ void zero() {
-        mp0 = p12 = f01 = make_float2(0.f, 0.f);
-        f2 = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) th[i] = 0.f;
-    }
-    // N, g0, g1, g2 arrive as broadcast pairs (both lanes equal)
-    __device__ __forceinline__ void add2(const float2 cm, const float2 cp, const float2 cb, const float2 cs0,
-                                         const float2 cs1, const float2 cs2, const P2GCoef<float, THERM> &q,
-                                         float2 NN, float2 G0, float2 G1, float2 G2) {
-        mp0 = __ffma2_rn(cm, NN, mp0);
-        p12 = __ffma2_rn(cp, NN, p12);
-        f01 = __ffma2_rn(cb, NN, f01);
-        f01 = __ffma2_rn(cs0, G0, f01);
-        f01 = __ffma2_rn(cs1, G1, f01);
-        f01 = __ffma2_rn(cs2, G2, f01);
-        f2 = fmaf(q.s[5], G2.x, fmaf(q.s[4], G1.x, fmaf(q.s[2], G0.x, fmaf(q.b[2], NN.x, f2))));
-        if constexpr (THERM) {
-            th[0] = fmaf(q.mcp, NN.x, th[0]);
-            th[1] = fmaf(q.mcpT, NN.x, th[1]);
-            th[2] = fmaf(q.mk, NN.x, th[2]);
-            th[3] = fmaf(q.VQ, NN.x, fmaf(q.qv[2], G2.x, fmaf(q.qv[1], G1.x, fmaf(q.qv[0], G0.x, th[3]))));
-        }
-    }
-    __device__ __forceinline__ float get(int ch) const {
-        switch (ch) {
-            case CH_M: return mp0.x;
-            case CH_P: return mp0.y;
-            case CH_P + 1: return p12.x;
-            case CH_P + 2: return p12.y;
-            case CH_F: return f01.x;
-            case CH_F + 1: return f01.y;
-            case CH_F + 2: return f2;
-            default: return th[ch - CH_MC];
-        }
-    }
-};
-
-constexpr int kCellThreads = 128;
-// launch shapes of the quadratic P2G and of the fused G2P (threads per
-// block, minimum resident blocks per SM for the register cap); the fused
-// G2P measured fastest at 2 x 256 (128 registers) against 1 x 256, 4 x 128,
-// 3 x 128, 3 x 256, 2 x 384 and 1 x 512
-constexpr int kMaxTileCells = 512;  // T^3 for the largest tile side, 8
-#ifndef EXG_P2G2_THREADS
-#define EXG_P2G2_THREADS 512
-#endif
-#ifndef EXG_P2G2_MINB
-#define EXG_P2G2_MINB 1
-#endif
+// launch shape of the fused G2P (threads per block, minimum resident blocks
+// per SM for the register cap): measured fastest at 2 x 256 (128 registers)
+// against 1 x 256, 4 x 128, 3 x 128, 3 x 256, 2 x 384 and 1 x 512
 #ifndef EXG_G2P_THREADS
 #define EXG_G2P_THREADS 256
 #endif
-// Quadratic momentum P2G with the z-slices split across threads, a bin's
-// three slices in adjacent threads (FP32 P2G 0.77 ms on the dam break
-// against 1.01 ms unsplit and 0.87 ms with the slices in separate thirds of
-// the block; FP64 1.47 against 2.51 ms unsplit)
-#ifndef EXG_P2G_SPLIT
-#define EXG_P2G_SPLIT 1
-#endif
-// L2 prefetch, at the start of each bin, of the first particle of the bin
-// the thread takes next (P2G 0.87-0.90 ms against 0.91 ms without)
-#ifndef EXG_P2G_PREFETCH
-#define EXG_P2G_PREFETCH 1
-#endif
-
 #ifndef EXG_G2P_MINB
 #define EXG_G2P_MINB 2
 #endif
-
-// Threads per block and register cap of the per-cell P2G: the 3-wide
-// quadratic accumulators fit 128 registers; one 512-thread block per SM (a
-// thread per bin of an 8^3 tile) measured fastest on the dam break, ahead
-// of 2 x 256, 4 x 128 and 1 x 256 with 255 registers.
-// Launch variants of the factorized momentum P2G (uniform quadratic and
-// cubic): rows per pass, threads per block and the minimum resident blocks
-// per SM (the register cap).  Variant 0 is the default; the autotuner
-// measures all kP2GVariants on the context's own particles and keeps the
-// fastest.  FP32 cubic holds a 4 x 4 slice (112 accumulators, one 256-thread
-// block per SM; half slices at 16 warps per SM measured 35 % slower); FP64
-// holds one or two rows.
-constexpr int kP2GVariants = 3;
-static_assert(kP2GVariants == EXG_NUM_VARIANTS, "the launchers dispatch EXG_NUM_VARIANTS P2G variants");
-// rows per pass, threads per block, minimum blocks per SM, lane map (0: a
-// warp takes one z-slice of 32 cells, 1: a cell's slices in adjacent
-// lanes), channel groups (2: mass and momentum apart from force)
-//   FP32 cubic:     (4, 256, 1, 0, 1)  (4, 256, 1, 1, 1)  (4, 256, 2, 0, 2)
-//   FP32 quadratic: (3, 512, 1, 0, 1)  (3, 512, 1, 1, 1)  (3, 256, 2, 0, 1)
-//   FP64 cubic:     (1, 512, 1, 1, 1)  (2, 256, 1, 1, 1)  (1, 512, 1, 0, 1)
-//   FP64 quadratic: (1, 512, 1, 1, 1)  (3, 256, 1, 1, 1)  (1, 512, 1, 0, 1)
-template <class R, int ORD, int V>
-struct P2GVar {
-    static constexpr int K = (sizeof(R) == 4 ? 0 : 2) + (ORD == 3 ? 0 : 1);
-    static constexpr int TAB[4][3][5] = {{{4, 256, 1, 0, 1}, {4, 256, 1, 1, 1}, {4, 256, 2, 0, 2}},
-                                         {{3, 512, 1, 0, 1}, {3, 512, 1, 1, 1}, {3, 256, 2, 0, 1}},
-                                         {{1, 512, 1, 1, 1}, {2, 256, 1, 1, 1}, {1, 512, 1, 0, 1}},
-                                         {{1, 512, 1, 1, 1}, {3, 256, 1, 1, 1}, {1, 512, 1, 0, 1}}};
-    static constexpr int ROWS = TAB[K][V][0], THREADS = TAB[K][V][1], MINB = TAB[K][V][2], MAP = TAB[K][V][3];
-    static constexpr int GROUPS = TAB[K][V][4];
-};
-
-template <class R, int ORD, bool THERM>
-struct P2GCfg {
-    static constexpr int W = P2GStc<ORD>::W;
-    static constexpr bool FACT = (ORD == 2 || ORD == 3) && !THERM;
-    // y rows of the stencil slice accumulated per pass (register budget)
-    static constexpr int ROWS = FACT ? P2GVar<R, (FACT ? ORD : 2), 0>::ROWS
-                                     : ((sizeof(R) == 8) ? 1 : (THERM ? (W == 4 ? 2 : 1) : W));
-    // quadratic momentum: the three z-slices of a bin's window go to three
-    // adjacent threads (FP32: one pass each, FP64: one pass per y row)
-    // instead of one thread walking them in turn, so the bin's particles are
-    // read by the three together and stay in L1
-    static constexpr bool SPLIT = EXG_P2G_SPLIT && ORD == 2 && !THERM;
-    static constexpr int THREADS = FACT ? P2GVar<R, (FACT ? ORD : 2), 0>::THREADS
-                                        : ((ORD == 2) ? EXG_P2G2_THREADS : kCellThreads);
-    static constexpr int MINB = FACT ? P2GVar<R, (FACT ? ORD : 2), 0>::MINB : ((ORD == 2) ? EXG_P2G2_MINB : 1);
-    static constexpr int MAP = FACT ? P2GVar<R, (FACT ? ORD : 2), 0>::MAP : 0;
-};
-
-// One tile of the per-cell P2G into its fixed-point node block (zeroed by
-// the caller) and from there to the tile's staging slot.
-template <class R, int ORD, bool THERM>
-__device__ __forceinline__ void p2g_tile(const SplineTables *tab, unsigned *acc_lo, int *acc_hi, const Params &P,
-                                         const Parts<R> &A, const int *active, const int *start, const int *cell_start,
-                                         const int32_t *perm, long long *staging, const R *sc, const R *grav, int w) {
-    constexpr int W = P2GCfg<R, ORD, THERM>::W;
-    constexpr int NCH = THERM ? CH_ALL : CH_MOM_END;
-    constexpr int ROWS = P2GCfg<R, ORD, THERM>::ROWS;
-    const int B = P.B, B3 = B * B * B, T = P.T, T3 = T * T * T;
-    const int t = active[w];
-    int tc[3];
-    tile_coords(P, t, tc);
-    const int s0 = start[t];
-    const int *cs = cell_start + (long long)w * (T3 + 1);
-    constexpr bool SPLIT = P2GCfg<R, ORD, THERM>::SPLIT;
-    // split: tasks (bin, slice) with the three slices of a bin in adjacent
-    // threads, so they read the bin's particles together and every thread of
-    // a 512-thread block takes exactly three tasks of an 8^3 tile
-    const int ntask = SPLIT ? W * T3 : T3, step = (int)blockDim.x;
-    for (int u = threadIdx.x; u < ntask; u += step) {
-        const int c = SPLIT ? u / W : u;
-        const int sz_lo = SPLIT ? u - c * W : 0, sz_hi = SPLIT ? sz_lo + 1 : W;
-        const int cnext = SPLIT ? (u + step) / W : u + step;
-        const int ka = cs[c], kb = cs[c + 1];
-        if (EXG_P2G_PREFETCH && sz_lo == 0 && cnext < T3) {
-            // L2 prefetch of the first particle of the bin this thread takes next
-            const int kn = cs[cnext];
-            if (kn < cs[cnext + 1]) {
-                const int pn = perm[s0 + kn];
-                auto pf = [](const void *q) { asm volatile("prefetch.global.L2 [%0];" ::"l"(q)); };
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    pf(A.x[d] + pn);
-                    pf(A.v[d] + pn);
-                }
-#pragma unroll
-                for (int c6 = 0; c6 < 6; ++c6) pf(A.sig[c6] + pn);
-                pf(A.mass + pn);
-                pf(A.vol + pn);
-                pf(A.phase + pn);
-            }
-        }
-        if (ka == kb) continue;
-        const int lx = c % T, ly = (c / T) % T, lz = c / (T * T);
-        const int iv[3] = {tc[0] * T + lx, tc[1] * T + ly, tc[2] * T + lz};
-        bool inter[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-            inter[d] = (ORD == 1) || P.periodic[d] ||
-                       (ORD == 2 ? (iv[d] >= 3 && iv[d] <= P.nc[d] - 3) : (iv[d] >= 3 && iv[d] <= P.nc[d] - 4));
-        for (int sz = sz_lo; sz < sz_hi; ++sz) {
-#pragma unroll
-            for (int sy0 = 0; sy0 < W; sy0 += ROWS) {
-                P2GAcc<R, THERM> acc[ROWS][W];
-#pragma unroll
-                for (int r = 0; r < ROWS; ++r)
-#pragma unroll
-                    for (int sx = 0; sx < W; ++sx) acc[r][sx].zero();
-                bool any = false;
-                for (int k = ka; k < kb; ++k) {
-                    const int p = perm[s0 + k];
-                    if (A.phase[p] != 0) continue;
-                    const double x[3] = {A.x[0][p], A.x[1][p], A.x[2][p]};
-                    AxisW<R, W> az;
-                    p2g_axis_weights<R, ORD>(*tab, P, 2, dual_x(P, 2, x[2]), iv[2], inter[2], az);
-                    const R wz = pick<W>(az.w, sz), dzw = pick<W>(az.dw, sz);
-                    if (wz == R(0) && dzw == R(0)) continue;
-                    any = true;
-                    AxisW<R, W> ax, ay;
-                    p2g_axis_weights<R, ORD>(*tab, P, 0, dual_x(P, 0, x[0]), iv[0], inter[0], ax);
-                    p2g_axis_weights<R, ORD>(*tab, P, 1, dual_x(P, 1, x[1]), iv[1], inter[1], ay);
-                    // every channel is deposited; the nodal kernel keeps
-                    // the ones the call asked for
-                    P2GCoef<R, THERM> q;
-                    q.m = A.mass[p];
-                    const R vol = A.vol[p];
-                    const bool slab = P.external_loads && x[0] > P.slab_lo[0] && x[0] < P.slab_hi[0] &&
-                                      x[1] > P.slab_lo[1] && x[1] < P.slab_hi[1] && x[2] > P.slab_lo[2] &&
-                                      x[2] < P.slab_hi[2];
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        q.mv[d] = q.m * A.v[d][p];
-                        q.b[d] = q.m * grav[d] + (slab ? (R)P.extforce[d] : R(0));
-                    }
-#pragma unroll
-                    for (int c6 = 0; c6 < 6; ++c6) q.s[c6] = -vol * A.sig[c6][p];
-                    if constexpr (THERM) {
-                        q.mcp = q.m * A.cp[p];
-                        q.mcpT = (R)(q.mcp * (A.T[p] - P.Tref));
-                        q.mk = q.m * A.kc[p];
-#pragma unroll
-                        for (int d = 0; d < 3; ++d) q.qv[d] = vol * A.q[d][p];
-                        q.VQ = vol * A.Q[p];
-                    }
-                    if constexpr (sizeof(R) == 4) {
-                        const float2 cm = make_float2(q.m, q.mv[0]), cp = make_float2(q.mv[1], q.mv[2]);
-                        const float2 cb = make_float2(q.b[0], q.b[1]);
-                        const float2 cs0 = make_float2(q.s[0], q.s[1]), cs1 = make_float2(q.s[1], q.s[3]),
-                                     cs2 = make_float2(q.s[2], q.s[4]);
-                        const float2 wzz = make_float2(wz, wz), dzz = make_float2(dzw, dzw);
-#pragma unroll
-                        for (int r = 0; r < ROWS; ++r) {
-                            const float2 wyy = make_float2(ay.w[sy0 + r], ay.w[sy0 + r]);
-                            const float2 dyy = make_float2(ay.dw[sy0 + r], ay.dw[sy0 + r]);
-                            const float2 wyz = __fmul2_rn(wyy, wzz), dyz = __fmul2_rn(dyy, wzz),
-                                         wdz = __fmul2_rn(wyy, dzz);
-#pragma unroll
-                            for (int sx = 0; sx < W; ++sx) {
-                                const float2 wxx = make_float2(ax.w[sx], ax.w[sx]);
-                                const float2 dxx = make_float2(ax.dw[sx], ax.dw[sx]);
-                                acc[r][sx].add2(cm, cp, cb, cs0, cs1, cs2, q, __fmul2_rn(wxx, wyz),
-                                                __fmul2_rn(dxx, wyz), __fmul2_rn(wxx, dyz), __fmul2_rn(wxx, wdz));
-                            }
-                        }
-                    } else {
-#pragma unroll
-                        for (int r = 0; r < ROWS; ++r) {
-                            const R wy = ay.w[sy0 + r], dyw = ay.dw[sy0 + r];
-                            const R wyz = wy * wz, dyz = dyw * wz, wdz = wy * dzw;
-#pragma unroll
-                            for (int sx = 0; sx < W; ++sx) {
-                                const R wx = ax.w[sx];
-                                acc[r][sx].add(q, wx * wyz, ax.dw[sx] * wyz, wx * dyz, wx * wdz);
-                            }
-                        }
-                    }
-                }
-                if (!any) continue;
-#pragma unroll
-                for (int r = 0; r < ROWS; ++r)
-#pragma unroll
-                    for (int sx = 0; sx < W; ++sx) {
-                        const int idx = ((lz + sz) * B + (ly + sy0 + r)) * B + (lx + sx);
-#pragma unroll
-                        for (int ch = 0; ch < NCH; ++ch)
-                            fx_add_r<R>(acc_lo, acc_hi, ch * B3 + idx, acc[r][sx].get(ch), sc[ch]);
-                    }
-            }
-        }
-    }
-    __syncthreads();
-    fx_store<R>(acc_lo, acc_hi, NCH * B3, staging + (long long)w * stg_stride<R>((long long)NCH * B3));
-    __syncthreads();
-}
-
-template <class R, int ORD, bool THERM>
-__global__ void __launch_bounds__(P2GCfg<R, ORD, THERM>::THREADS, P2GCfg<R, ORD, THERM>::MINB)
-    k_p2g_cell(Params P, Parts<R> A, const int *active, const int *start, const int *cell_start, const int32_t *perm,
-               long long *staging, Ctl *ctl, int flags) {
-    constexpr int NCH = THERM ? CH_ALL : CH_MOM_END;
-    __shared__ int s_item;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    SplineTables *tab = reinterpret_cast<SplineTables *>(smraw);
-    const int B3 = P.B * P.B * P.B;
-    unsigned *acc_lo = reinterpret_cast<unsigned *>(smraw + ((sizeof(SplineTables) + 15) & ~15));
-    int *acc_hi = reinterpret_cast<int *>(acc_lo + NCH * B3 * fx_lo_words<R>());
-    load_tables(tab);
-    R sc[NCH];
-#pragma unroll
-    for (int c = 0; c < NCH; ++c) sc[c] = (R)ctl->scale[c];
-    (void)flags;  // every channel is deposited; the nodal kernel keeps the requested ones
-    R grav[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) grav[d] = (R)P.gravity[d];
-    const int nitems = ctl->n_active_tiles;
-    for (;;) {
-        // tiles are taken in turn from a device counter: blocks that drew
-        // light tiles take more of them
-        if (threadIdx.x == 0) s_item = atomicAdd(&ctl->next_p2g, 1);
-        fx_zero<R>(acc_lo, acc_hi, NCH * B3);
-        __syncthreads();
-        const int w = s_item;
-        if (w >= nitems) break;
-        p2g_tile<R, ORD, THERM>(tab, acc_lo, acc_hi, P, A, active, start, cell_start, perm, staging, sc, grav, w);
-    }
-}
-
-// ---------------------------------------------------------------- K2 factorized P2G
-// Momentum P2G of uniform quadratic (nearest-node bins) and cubic (cells)
-// B-splines with the deposit of deposit_onto_grid_momentum
-// (mpm_particle_grid_ops.cpp:484-577) in factorized form.  With
-// N = wx wy wz and grad N = (dwx wy wz, wx dwy wz, wx wy dwz), s_dj =
-// -V sigma_dj and b_d = m g_d (+ f_ext,d inside the force slab):
-//   m N          = wx (wy (m wz))
-//   m v_d N      = wx (wy (m v_d wz))
-//   f_d          = wx (wy A_d + dwy B_d) + dwx (wy C_d),
-//   A_d = b_d wz + s_d2 dwz,  B_d = s_d1 wz,  C_d = s_d0 wz,
-// so a node costs 4 packed FP32 FMAs and 2 scalar ones (10 FMAs in FP64)
-// instead of forming N and grad N.  Tasks are (cell, z-slice, row group):
-// the W x NPASS tasks of a cell sit in adjacent threads, read the cell's
-// particles together (they stay in L1) and each accumulates ROWS rows of its
-// slice in registers, then adds the cell's sums to the tile's fixed-point
-// node block.  Every node's register sum runs over the cell's particles in
-// storage order with the same expression whatever ROWS and the block size
-// are, so all launch variants give bit-identical results.
-template <class R, int ROWS>
-struct FactRow;  // row terms (wy and dwy folded into the z-level terms)
-template <int ROWS>
-struct FactRow<float, ROWS> {
-    float2 mp0, p12, a01, c01;
-    float a2, c2;
-};
-template <int ROWS>
-struct FactRow<double, ROWS> {
-    double m, p[3], a[3], c[3];
-};
-
-template <class R>
-struct FactAcc;
-template <>
-struct FactAcc<float> {
-    float2 mp0, p12, f01;
-    float f2;
-    __device__ __forceinline__ void zero() {
-        mp0 = p12 = f01 = make_float2(0.f, 0.f);
-        f2 = 0.f;
-    }
-    // GRP 0: every channel; 1: mass and momentum; 2: force (the same
-    // operations on each channel in every case)
-    template <int GRP = 0>
-    __device__ __forceinline__ void add(const FactRow<float, 1> &r, float2 wxx, float2 dxx) {
-        if (GRP != 2) {
-            mp0 = __ffma2_rn(wxx, r.mp0, mp0);
-            p12 = __ffma2_rn(wxx, r.p12, p12);
-        }
-        if (GRP != 1) {
-            f01 = __ffma2_rn(wxx, r.a01, f01);
-            f01 = __ffma2_rn(dxx, r.c01, f01);
-            f2 = fmaf(wxx.x, r.a2, f2);
-            f2 = fmaf(dxx.x, r.c2, f2);
-        }
-    }
-    __device__ __forceinline__ float get(int ch) const {
-        switch (ch) {
-            case CH_M: return mp0.x;
-            case CH_P: return mp0.y;
-            case CH_P + 1: return p12.x;
-            case CH_P + 2: return p12.y;
-            case CH_F: return f01.x;
-            case CH_F + 1: return f01.y;
-            default: return f2;
-        }
-    }
-};
-template <>
-struct FactAcc<double> {
-    double c[CH_MOM_END];
-    __device__ __forceinline__ void zero() {
-#pragma unroll
-        for (int i = 0; i < CH_MOM_END; ++i) c[i] = 0.0;
-    }
-    template <int GRP = 0>
-    __device__ __forceinline__ void add(const FactRow<double, 1> &r, double wx, double dwx) {
-        if (GRP != 2) {
-            c[CH_M] = fma(wx, r.m, c[CH_M]);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) c[CH_P + d] = fma(wx, r.p[d], c[CH_P + d]);
-        }
-        if (GRP != 1) {
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                c[CH_F + d] = fma(wx, r.a[d], c[CH_F + d]);
-                c[CH_F + d] = fma(dwx, r.c[d], c[CH_F + d]);
-            }
-        }
-    }
-    __device__ __forceinline__ double get(int ch) const { return c[ch]; }
-};
-
-// z-level terms of one particle for one node plane
-template <class R>
-struct FactZ {
-    R m, p[3], a[3], b[3], c[3];
-};
-
-template <class R>
-__device__ __forceinline__ FactRow<R, 1> fact_row(const FactZ<R> &z, R wy, R dwy) {
-    FactRow<R, 1> r;
-    if constexpr (sizeof(R) == 4) {
-        const float2 wyy = make_float2(wy, wy), dyy = make_float2(dwy, dwy);
-        r.mp0 = __fmul2_rn(wyy, make_float2(z.m, z.p[0]));
-        r.p12 = __fmul2_rn(wyy, make_float2(z.p[1], z.p[2]));
-        r.a01 = __ffma2_rn(dyy, make_float2(z.b[0], z.b[1]), __fmul2_rn(wyy, make_float2(z.a[0], z.a[1])));
-        r.a2 = fmaf(dwy, z.b[2], wy * z.a[2]);
-        r.c01 = __fmul2_rn(wyy, make_float2(z.c[0], z.c[1]));
-        r.c2 = wy * z.c[2];
-    } else {
-        r.m = wy * z.m;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            r.p[d] = wy * z.p[d];
-            r.a[d] = fma(dwy, z.b[d], wy * z.a[d]);
-            r.c[d] = wy * z.c[d];
-        }
-    }
-    return r;
-}
-
-// Weight and derivative of one slot (the task's z-slice): the interior piece
-// of that slot alone, or the boundary-aware tables.  s is warp-uniform (the
-// task mapping gives a warp one slice), so the switch does not diverge.
-template <class R, int ORD>
-__device__ __forceinline__ void slot_weight(const SplineTables &tab, const Params &P, int d, double x, int i,
-                                            bool interior, R f, int s, R &w, R &dw) {
-    const R dxinv = (R)P.dxi[d];
-    if (interior) {
-        if constexpr (sizeof(R) == 4) {
-            slot_weight_f32(ORD, f, s, w, dw);
-        } else if constexpr (ORD == 3) {
-            const R o6 = (R)kOneBySix, t3 = (R)kTwoByThree, f3 = (R)kFourByThree;
-            const R z = f + R(1 - s), z2 = z * z;
-            switch (s) {
-                case 0: w = fma(-o6, z2 * z, fma(R(1), z2, fma(R(-2), z, f3))); dw = fma(R(-0.5), z2, fma(R(2), z, R(-2))); break;
-                case 1: w = fma(R(0.5), z2 * z, fma(R(-1), z2, fma(R(0), z, t3))); dw = fma(R(1.5), z2, fma(R(-2), z, R(0))); break;
-                case 2: w = fma(R(-0.5), z2 * z, fma(R(-1), z2, fma(R(0), z, t3))); dw = fma(R(-1.5), z2, fma(R(-2), z, R(0))); break;
-                default: w = fma(o6, z2 * z, fma(R(1), z2, fma(R(2), z, f3))); dw = fma(R(0.5), z2, fma(R(2), z, R(2))); break;
-            }
-        } else {
-            const R z = f + R(1 - s);
-            switch (s) {
-                case 0: w = fma(R(0.5), z * z, fma(R(-1.5), z, R(1.125))); dw = z - R(1.5); break;
-                case 1: w = fma(R(-1), z * z, fma(R(0), z, R(0.75))); dw = R(-2) * z; break;
-                default: w = fma(R(0.5), z * z, fma(R(1.5), z, R(1.125))); dw = z + R(1.5); break;
-            }
-        }
-        dw *= dxinv;
-    } else {
-        AxisW<R, P2GStc<ORD>::W> a;
-        p2g_axis_weights<R, ORD>(tab, P, d, x, i, false, a);
-        w = pick<P2GStc<ORD>::W>(a.w, s);
-        dw = pick<P2GStc<ORD>::W>(a.dw, s);
-    }
-}
 
 // Weights of all slots of one axis: interior pieces from the offset f, the
 // tables elsewhere.
@@ -1518,390 +993,7 @@ __device__ __forceinline__ void fact_axis_weights(const SplineTables &tab, const
         p2g_axis_weights<R, ORD>(tab, P, d, x, i, false, a);
 }
 
-// The particles ka..kb-1 of one cell (bin) into a task's accumulators: for
-// each particle the z weight of the task's slice first (a zero slice weight
-// and derivative skip it), then the x and y weights, the particle's
-// z-factored terms, and per y row of the task a packed FMA per node and
-// channel pair.  Returns whether any particle contributed.
-template <class R, int ORD, int ROWS, int MAP, int GRP = 0>
-__device__ __forceinline__ bool fact_deposit_cell(const SplineTables *tab, const Params &P, const Parts<R> &A,
-                                                  const int32_t *perm, int s0, int ka, int kb, const int iv[3],
-                                                  const bool inter[3], const double xo[3], int sz, int rg,
-                                                  const R *grav, FactAcc<R> (&acc)[ROWS][P2GStc<ORD>::W]) {
-    constexpr int W = P2GStc<ORD>::W;
-    constexpr int NPASS = W / ROWS;
-    bool any = false;
-    for (int k = ka; k < kb; ++k) {
-        const int p = perm[s0 + k];
-        if (A.phase[p] != 0) continue;
-        const double x[3] = {A.x[0][p], A.x[1][p], A.x[2][p]};
-        double xw[3];
-        R f[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            xw[d] = dual_x(P, d, x[d]);
-            f[d] = (R)((xw[d] - xo[d]) * P.dxi[d]);
-        }
-        R wz, dwz;
-        if (MAP == 0) {
-            slot_weight<R, ORD>(*tab, P, 2, xw[2], iv[2], inter[2], f[2], sz, wz, dwz);
-        } else {
-            AxisW<R, W> az;
-            fact_axis_weights<R, ORD>(*tab, P, 2, xw[2], iv[2], inter[2], f[2], az);
-            wz = pick<W>(az.w, sz);
-            dwz = pick<W>(az.dw, sz);
-        }
-        if (wz == R(0) && dwz == R(0)) continue;
-        any = true;
-        AxisW<R, W> ax, ay;
-        fact_axis_weights<R, ORD>(*tab, P, 0, xw[0], iv[0], inter[0], f[0], ax);
-        fact_axis_weights<R, ORD>(*tab, P, 1, xw[1], iv[1], inter[1], f[1], ay);
-        const R m = A.mass[p], vol = A.vol[p];
-        const bool slab = P.external_loads && x[0] > P.slab_lo[0] && x[0] < P.slab_hi[0] && x[1] > P.slab_lo[1] &&
-                          x[1] < P.slab_hi[1] && x[2] > P.slab_lo[2] && x[2] < P.slab_hi[2];
-        R sg[6];
-#pragma unroll
-        for (int c6 = 0; c6 < 6; ++c6) sg[c6] = -vol * A.sig[c6][p];
-        // rows of the symmetric stress in packed XX XY XZ YY YZ ZZ order
-        const R s0r[3] = {sg[0], sg[1], sg[2]}, s1r[3] = {sg[1], sg[3], sg[4]}, s2r[3] = {sg[2], sg[4], sg[5]};
-        FactZ<R> z;
-        z.m = m * wz;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const R bd = fma(m, grav[d], slab ? (R)P.extforce[d] : R(0));
-            const R sd0 = d == 0 ? s0r[0] : (d == 1 ? s1r[0] : s2r[0]);
-            const R sd1 = d == 0 ? s0r[1] : (d == 1 ? s1r[1] : s2r[1]);
-            const R sd2 = d == 0 ? s0r[2] : (d == 1 ? s1r[2] : s2r[2]);
-            z.p[d] = (m * A.v[d][p]) * wz;
-            z.a[d] = fma(sd2, dwz, bd * wz);
-            z.b[d] = sd1 * wz;
-            z.c[d] = sd0 * wz;
-        }
-#pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-            const int sy = rg * ROWS + r;
-            const R wy = NPASS == 1 ? ay.w[r] : pick<W>(ay.w, sy);
-            const R dwy = NPASS == 1 ? ay.dw[r] : pick<W>(ay.dw, sy);
-            const FactRow<R, 1> row = fact_row<R>(z, wy, dwy);
-#pragma unroll
-            for (int sx = 0; sx < W; ++sx) {
-                if constexpr (sizeof(R) == 4)
-                    acc[r][sx].template add<GRP>(row, make_float2(ax.w[sx], ax.w[sx]),
-                                                 make_float2(ax.dw[sx], ax.dw[sx]));
-                else
-                    acc[r][sx].template add<GRP>(row, ax.w[sx], ax.dw[sx]);
-            }
-        }
-    }
-    return any;
-}
-
-// L2 prefetch of the first particle of cell c, if it has one.
-template <class R>
-__device__ __forceinline__ void prefetch_cell_head(const Parts<R> &A, const int32_t *perm, int s0, const int *cs,
-                                                   int c) {
-    const int kn = cs[c];
-    if (kn < cs[c + 1]) {
-        const int pn = perm[s0 + kn];
-        auto pf = [](const void *q) { asm volatile("prefetch.global.L2 [%0];" ::"l"(q)); };
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            pf(A.x[d] + pn);
-            pf(A.v[d] + pn);
-        }
-#pragma unroll
-        for (int c6 = 0; c6 < 6; ++c6) pf(A.sig[c6] + pn);
-        pf(A.mass + pn);
-        pf(A.vol + pn);
-        pf(A.phase + pn);
-    }
-}
-
-template <class R, int ORD>
-__device__ __forceinline__ void cell_frame(const Params &P, const int tc[3], int lx, int ly, int lz, int iv[3],
-                                           bool inter[3], double xo[3]) {
-    const int T = P.T;
-    iv[0] = tc[0] * T + lx;
-    iv[1] = tc[1] * T + ly;
-    iv[2] = tc[2] * T + lz;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        inter[d] = P.periodic[d] ||
-                   (ORD == 2 ? (iv[d] >= 3 && iv[d] <= P.nc[d] - 3) : (iv[d] >= 3 && iv[d] <= P.nc[d] - 4));
-        xo[d] = P.plo[d] + iv[d] * P.dx[d];  // the cell's (cubic) or bin node's (quadratic) coordinate
-    }
-}
-
-// One tile of the factorized P2G, one task per (cell, z-slice, row group,
-// channel group): the task's ROWS x W node block accumulates the cell's
-// particles in registers and is added to the tile's fixed-point block after
-// the cell.  With GROUPS = 2 a cell's mass and momentum (4 channels, no
-// gradients, no stress) and its force (3 channels) go to separate tasks:
-// each holds at most 64 accumulators instead of 112, so two blocks fit an
-// SM, for about the same instructions; each channel's operations are the
-// same as with GROUPS = 1, so the results are the same bits.
-template <class R, int ORD, int ROWS, int MAP, int GROUPS = 1>
-__device__ __forceinline__ void p2g_tile_fact(const SplineTables *tab, unsigned *acc_lo, int *acc_hi, const Params &P,
-                                              const Parts<R> &A, const int *active, const int *start,
-                                              const int *cell_start, const int32_t *perm, long long *staging,
-                                              const R *sc, const R *grav, int w) {
-    constexpr int W = P2GStc<ORD>::W;
-    static_assert(W % ROWS == 0, "rows per pass must divide the stencil width");
-    constexpr int NPASS = W / ROWS, LANES = W * NPASS * GROUPS, NCH = CH_MOM_END;
-    const int B = P.B, B3 = B * B * B, T = P.T, T3 = T * T * T;
-    const int t = active[w];
-    int tc[3];
-    tile_coords(P, t, tc);
-    const int s0 = start[t];
-    const int *cs = cell_start + (long long)w * (T3 + 1);
-    // The tile's non-empty cells, in cell order (a block-wide compaction), so
-    // that no lane walks an empty cell: at a body's surface half the cells
-    // of a tile can be empty.  Cells keep their own sums, and the fixed-point
-    // adds do not depend on the order, so the results do not change.
-    __shared__ int s_cells[kMaxTileCells];
-    __shared__ int s_scan[34];
-    int ncomp;
-    {
-        const int per = (T3 + (int)blockDim.x - 1) / (int)blockDim.x, c0 = (int)threadIdx.x * per;
-        int cnt = 0;
-        for (int k = 0; k < per; ++k) {
-            const int cc = c0 + k;
-            cnt += (cc < T3 && cs[cc] < cs[cc + 1]) ? 1 : 0;
-        }
-        int off = block_exclusive_scan(cnt, &ncomp, s_scan);
-        for (int k = 0; k < per; ++k) {
-            const int cc = c0 + k;
-            if (cc < T3 && cs[cc] < cs[cc + 1]) s_cells[off++] = cc;
-        }
-        __syncthreads();
-    }
-    // task u -> (cell index in the compacted list, sub) with sub = (z-slice,
-    // row group, channel group).  MAP 0: warp u / 32 takes one sub of 32
-    // consecutive listed cells, so the slice and the channel group are
-    // warp-uniform (one z weight evaluated, no divergence); the LANES warps
-    // of a group of 32 cells are consecutive and run together (the cells'
-    // particles stay in L1).  MAP 1: a cell's LANES tasks sit in adjacent
-    // lanes, which read each particle with one load.
-    const int nlist = MAP == 0 ? ((ncomp + 31) & ~31) : ncomp;
-    const int ntask = LANES * nlist, step = (int)blockDim.x;
-    auto task = [&](int uu, int &cc, int &ss) {
-        if (MAP == 0) {
-            const int wi = uu >> 5, g = wi / LANES;
-            ss = wi - g * LANES;
-            cc = g * 32 + (uu & 31);
-        } else {
-            cc = uu / LANES;
-            ss = uu - cc * LANES;
-        }
-    };
-    for (int u = threadIdx.x; u < ntask; u += step) {
-        int ci, sub;
-        task(u, ci, sub);
-        if (ci >= ncomp) continue;
-        const int c = s_cells[ci];
-        const int grp = GROUPS == 1 ? 0 : sub % GROUPS, sp = sub / GROUPS;
-        const int sz = sp / NPASS, rg = sp - sz * NPASS;
-        const int ka = cs[c], kb = cs[c + 1];
-        if (EXG_P2G_PREFETCH && sub == 0) {
-            // L2 prefetch of the first particle of the cell this thread takes next
-            const int un = u + step;
-            int cn = 0, sn = 1;
-            if (un < ntask) task(un, cn, sn);
-            if (un < ntask && sn == 0 && cn < ncomp) prefetch_cell_head(A, perm, s0, cs, s_cells[cn]);
-        }
-        const int lx = c % T, ly = (c / T) % T, lz = c / (T * T);
-        int iv[3];
-        bool inter[3];
-        double xo[3];
-        cell_frame<R, ORD>(P, tc, lx, ly, lz, iv, inter, xo);
-        // each branch has its own accumulators (only its channels live)
-        auto cell_task = [&](auto grp_tag) {
-            constexpr int G = decltype(grp_tag)::value;
-            constexpr int CH0 = G == 2 ? CH_F : 0, CH1 = G == 1 ? CH_F : NCH;
-            FactAcc<R> acc[ROWS][W];
-#pragma unroll
-            for (int r = 0; r < ROWS; ++r)
-#pragma unroll
-                for (int sx = 0; sx < W; ++sx) acc[r][sx].zero();
-            if (!fact_deposit_cell<R, ORD, ROWS, MAP, G>(tab, P, A, perm, s0, ka, kb, iv, inter, xo, sz, rg, grav,
-                                                         acc))
-                return;
-#pragma unroll
-            for (int r = 0; r < ROWS; ++r)
-#pragma unroll
-                for (int sx = 0; sx < W; ++sx) {
-                    const int idx = ((lz + sz) * B + (ly + rg * ROWS + r)) * B + (lx + sx);
-#pragma unroll
-                    for (int ch = CH0; ch < CH1; ++ch)
-                        fx_add_r<R>(acc_lo, acc_hi, ch * B3 + idx, acc[r][sx].get(ch), sc[ch]);
-                }
-        };
-        if (GROUPS == 1)
-            cell_task(std::integral_constant<int, 0>{});
-        else if (grp == 0)
-            cell_task(std::integral_constant<int, 1>{});
-        else
-            cell_task(std::integral_constant<int, 2>{});
-    }
-    __syncthreads();
-    fx_store<R>(acc_lo, acc_hi, NCH * B3, staging + (long long)w * stg_stride<R>((long long)NCH * B3));
-    __syncthreads();
-}
-
-// Segments a row of a tile is cut into for p2g_tile_xrun (1: whole rows;
-// half rows measured no faster: the block's closing barrier waits for the
-// slowest segment either way).
-constexpr int kXRunParts = 1;
-
-// One tile of the factorized P2G, one task per (segment of T / kXRunParts
-// cells along x, z-slice, row group): the task walks its segment's cells in
-// x order with a window of W node columns in registers.  Once cell cx is
-// done, no later cell of the segment reaches node column cx, so that column
-// alone goes to the tile's fixed-point block and the window moves by one
-// column; the last W - 1 columns go after the segment.  Per cell one column
-// of ROWS x 7 values is converted and added instead of W columns.
-template <class R, int ORD, int ROWS, int MAP>
-__device__ __forceinline__ void p2g_tile_xrun(const SplineTables *tab, unsigned *acc_lo, int *acc_hi, const Params &P,
-                                              const Parts<R> &A, const int *active, const int *start,
-                                              const int *cell_start, const int32_t *perm, long long *staging,
-                                              const R *sc, const R *grav, int w) {
-    constexpr int W = P2GStc<ORD>::W;
-    static_assert(W % ROWS == 0, "rows per pass must divide the stencil width");
-    constexpr int NPASS = W / ROWS, LANES = W * NPASS, NCH = CH_MOM_END;
-    const int B = P.B, B3 = B * B * B, T = P.T, T2 = T * T, T3 = T2 * T;
-    const int SL = T / kXRunParts, NSEG = T2 * kXRunParts;  // cells per segment, segments per tile
-    const int t = active[w];
-    int tc[3];
-    tile_coords(P, t, tc);
-    const int s0 = start[t];
-    const int *cs = cell_start + (long long)w * (T3 + 1);
-    // task u -> (segment, z-slice, row group); MAP 0: a warp takes one
-    // (z-slice, row group) of 32 segments (warp-uniform slice), MAP 1: a
-    // segment's LANES tasks in adjacent lanes
-    const int groups = (NSEG + 31) >> 5;
-    const int ntask = MAP == 0 ? groups * 32 * LANES : NSEG * LANES, step = (int)blockDim.x;
-    for (int u = threadIdx.x; u < ntask; u += step) {
-        int seg, sub;
-        if (MAP == 0) {
-            const int wi = u >> 5, g = wi / LANES;
-            sub = wi - g * LANES;
-            seg = g * 32 + (u & 31);
-        } else {
-            seg = u / LANES;
-            sub = u - seg * LANES;
-        }
-        if (seg >= NSEG) continue;
-        const int sz = sub / NPASS, rg = sub - sz * NPASS;
-        const int row = seg / kXRunParts, x0 = (seg - row * kXRunParts) * SL;
-        const int ly = row % T, lz = row / T;
-        const int c0 = row * T + x0;  // first cell of the segment (x fastest)
-        FactAcc<R> acc[ROWS][W];
-#pragma unroll
-        for (int r = 0; r < ROWS; ++r)
-#pragma unroll
-            for (int sx = 0; sx < W; ++sx) acc[r][sx].zero();
-        unsigned dirty = 0;  // bit j: window column j holds contributions
-        const int ybase = (lz + sz) * B + ly + rg * ROWS;
-        auto flush = [&](int j, int col) {
-#pragma unroll
-            for (int r = 0; r < ROWS; ++r) {
-                const int idx = (ybase + r) * B + col;
-#pragma unroll
-                for (int ch = 0; ch < NCH; ++ch) {
-                    R v;
-                    switch (j) {  // j is a compile-time constant at every call
-                        case 0: v = acc[r][0].get(ch); break;
-                        case 1: v = acc[r][1 % W].get(ch); break;
-                        case 2: v = acc[r][2 % W].get(ch); break;
-                        default: v = acc[r][W - 1].get(ch); break;
-                    }
-                    fx_add_r<R>(acc_lo, acc_hi, ch * B3 + idx, v, sc[ch]);
-                }
-            }
-        };
-        for (int k = 0; k < SL; ++k) {
-            const int cx = x0 + k, c = c0 + k;
-            const int ka = cs[c], kb = cs[c + 1];
-            if (EXG_P2G_PREFETCH && k + 1 < SL && sub == 0) prefetch_cell_head(A, perm, s0, cs, c + 1);
-            if (ka < kb) {
-                int iv[3];
-                bool inter[3];
-                double xo[3];
-                cell_frame<R, ORD>(P, tc, cx, ly, lz, iv, inter, xo);
-                if (fact_deposit_cell<R, ORD, ROWS, MAP>(tab, P, A, perm, s0, ka, kb, iv, inter, xo, sz, rg, grav,
-                                                         acc))
-                    dirty |= (1u << W) - 1u;
-            }
-            if (dirty & 1u) flush(0, cx);
-            // the window moves one column along x
-#pragma unroll
-            for (int r = 0; r < ROWS; ++r) {
-#pragma unroll
-                for (int j = 0; j + 1 < W; ++j) acc[r][j] = acc[r][j + 1];
-                acc[r][W - 1].zero();
-            }
-            dirty >>= 1;
-        }
-#pragma unroll
-        for (int j = 0; j + 1 < W; ++j)
-            if (dirty & (1u << j)) flush(j, x0 + SL + j);
-    }
-    __syncthreads();
-    fx_store<R>(acc_lo, acc_hi, NCH * B3, staging + (long long)w * stg_stride<R>((long long)NCH * B3));
-    __syncthreads();
-}
-
-// FP64 cubic tasks walk rows of cells (p2g_tile_xrun): its fixed-point
-// adds are returning 64-bit atomics, and the walk converts and adds a third
-// as many values (FP64 P2G 3.46 -> 2.97 ms on the 9 M-particle spheres).
-// FP32 cubic and all quadratic tasks take one cell (bin) each
-// (p2g_tile_fact): the FP32 adds are cheap, and the per-cell walk keeps
-// more tasks per thread to even out uneven cells (1.66 against 1.69 ms).
-// Every launch variant of one precision and order uses the same walk, so
-// the register sums and hence the results are the same for all of them.
-template <class R, int ORD, int ROWS, int MAP, int GROUPS = 1>
-__device__ __forceinline__ void p2g_tile_factorized(const SplineTables *tab, unsigned *acc_lo, int *acc_hi,
-                                                    const Params &P, const Parts<R> &A, const int *active,
-                                                    const int *start, const int *cell_start, const int32_t *perm,
-                                                    long long *staging, const R *sc, const R *grav, int w) {
-    if constexpr (ORD == 3 && sizeof(R) == 8)
-        p2g_tile_xrun<R, ORD, ROWS, MAP>(tab, acc_lo, acc_hi, P, A, active, start, cell_start, perm, staging, sc,
-                                         grav, w);
-    else
-        p2g_tile_fact<R, ORD, ROWS, MAP, GROUPS>(tab, acc_lo, acc_hi, P, A, active, start, cell_start, perm,
-                                                 staging, sc, grav, w);
-}
-
-template <class R, int ORD, int V>
-__global__ void __launch_bounds__(P2GVar<R, ORD, V>::THREADS, P2GVar<R, ORD, V>::MINB)
-    k_p2g_fact(Params P, Parts<R> A, const int *active, const int *start, const int *cell_start, const int32_t *perm,
-               long long *staging, Ctl *ctl) {
-    constexpr int NCH = CH_MOM_END;
-    __shared__ int s_item;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    SplineTables *tab = reinterpret_cast<SplineTables *>(smraw);
-    const int B3 = P.B * P.B * P.B;
-    unsigned *acc_lo = reinterpret_cast<unsigned *>(smraw + ((sizeof(SplineTables) + 15) & ~15));
-    int *acc_hi = reinterpret_cast<int *>(acc_lo + NCH * B3 * fx_lo_words<R>());
-    load_tables(tab);
-    R sc[NCH];
-#pragma unroll
-    for (int c = 0; c < NCH; ++c) sc[c] = (R)ctl->scale[c];
-    R grav[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) grav[d] = (R)P.gravity[d];
-    const int nitems = ctl->n_active_tiles;
-    for (;;) {
-        // tiles are taken in turn from a device counter
-        if (threadIdx.x == 0) s_item = atomicAdd(&ctl->next_p2g, 1);
-        fx_zero<R>(acc_lo, acc_hi, NCH * B3);
-        __syncthreads();
-        const int w = s_item;
-        if (w >= nitems) break;
-        p2g_tile_factorized<R, ORD, P2GVar<R, ORD, V>::ROWS, P2GVar<R, ORD, V>::MAP, P2GVar<R, ORD, V>::GROUPS>(
-            tab, acc_lo, acc_hi, P, A, active, start, cell_start, perm, staging, sc, grav, w);
-    }
-}
+#include "exg_p2g.cuh"
 
 // Domain-wall BCs of one node (nodal_bcs, nodal_data_ops.cpp:663-766),
 // UDF walls (apply_udf_nodal_bcs, :1061-1175) and level-set bodies
@@ -2055,7 +1147,8 @@ __device__ __forceinline__ void nodes_tile(const Params &P, const Nodes<R> &Nd, 
                                            const int *slot, const long long *staging, const double *isc, double dt,
                                            int mode, int flags, int w, unsigned &status) {
     constexpr int NCH = THERM ? CH_ALL : CH_MOM_END;
-    const int B = P.B, B3 = B * B * B, T = P.T;
+    const int B = P.B, T = P.T;
+    const int zs = P.tshift - P.pshift, parts = 1 << P.pshift;  // log2 of an item's z planes, items per tile
     const int t = tiles ? tiles[w] : w;
     int tc[3];
     tile_coords(P, t, tc);
@@ -2112,11 +1205,15 @@ __device__ __forceinline__ void nodes_tile(const Params &P, const Nodes<R> &Nd, 
                     const int lz = a ? l2[2] : l1[2], ly = b2 ? l2[1] : l1[1], lx = c2 ? l2[0] : l1[0];
                     const int sl = slot[(sz * P.ntile[1] + sy) * P.ntile[0] + sx];
                     if (sl < 0) continue;
-                    const long long nv = (long long)NCH * B3;
-                    const long long *blk = staging + (long long)sl * stg_stride<R>(nv);
-                    const long long off = ((long long)lz * B + ly) * B + lx;
+                    const int nv = p2g_values<THERM>(P);
+                    // the tile's items whose node planes hold plane lz (item s: planes s SZ .. s SZ + Bz - 1)
+                    const int p1 = min(parts - 1, lz >> zs);
+                    for (int s = lz >= P.Bz ? ((lz - P.Bz) >> zs) + 1 : 0; s <= p1; ++s) {
+                        const long long *blk = staging + (((long long)sl << P.pshift) + s) * stg_stride<R>(nv);
+                        const long long off = (long long)(lz - (s << zs)) * P.PS + ly * B + lx;
 #pragma unroll
-                    for (int c = 0; c < NCH; ++c) accv[c].add(blk, nv, off + (long long)c * B3);
+                        for (int c = 0; c < NCH; ++c) accv[c].add(blk, nv, off + (long long)c * (P.PS * P.Bz));
+                    }
                 }
         const long long ni = ((long long)nid[2] * P.nn[1] + nid[1]) * P.nn[0] + nid[0];
         double m = accv[CH_M].value() * isc[CH_M];
@@ -4049,45 +3146,36 @@ __global__ void __launch_bounds__(kBatchThreads) k_bb_copy_lost(const SceneDesc<
     copy_particle<R>(dr[s].A, i, Bo, j, temp != 0);
 }
 
-template <class R, int ORD, bool THERM>
-__global__ void __launch_bounds__(P2GCfg<R, ORD, THERM>::THREADS, P2GCfg<R, ORD, THERM>::MINB)
-    k_p2g_batch(const SceneDesc<R> *__restrict__ descs, BatchCtl *b, int B3) {
-    constexpr int NCH = THERM ? CH_ALL : CH_MOM_END;
-    __shared__ int s_item, s_scene;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    SplineTables *tab = reinterpret_cast<SplineTables *>(smraw);
-    unsigned *acc_lo = reinterpret_cast<unsigned *>(smraw + ((sizeof(SplineTables) + 15) & ~15));
-    int *acc_hi = reinterpret_cast<int *>(acc_lo + NCH * B3 * fx_lo_words<R>());
-    load_tables(tab);
-    const int ns = b->nscenes, total = b->pre_active[ns];
-    int cur = -1;
-    R sc[NCH], grav[3];
-    for (;;) {
-        if (threadIdx.x == 0) {
-            const int i = atomicAdd(&b->next_p2g, 1);
-            s_item = i;
-            s_scene = i < total ? scene_of(b->pre_active, ns, i) : -1;
-        }
-        fx_zero<R>(acc_lo, acc_hi, NCH * B3);
-        __syncthreads();
-        const int i = s_item, s = s_scene;
-        if (i >= total) break;
-        const SceneDesc<R> &sd = descs[s];
-        if (s != cur) {
-            cur = s;
-#pragma unroll
-            for (int c = 0; c < NCH; ++c) sc[c] = (R)sd.ctl->scale[c];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) grav[d] = (R)sd.P.gravity[d];
-        }
-        if constexpr (P2GCfg<R, ORD, THERM>::FACT)
-            p2g_tile_factorized<R, ORD, P2GCfg<R, ORD, THERM>::ROWS, P2GCfg<R, ORD, THERM>::MAP>(
-                tab, acc_lo, acc_hi, sd.P, sd.A, sd.active, sd.start, sd.cell_start, sd.perm, sd.staging, sc, grav,
-                i - b->pre_active[s]);
-        else
-            p2g_tile<R, ORD, THERM>(tab, acc_lo, acc_hi, sd.P, sd.A, sd.active, sd.start, sd.cell_start, sd.perm,
-                                    sd.staging, sc, grav, i - b->pre_active[s]);
+// Items of all scenes of a batch, taken in turn from one device counter.
+template <class R>
+struct P2GBatchSrc {
+    const SceneDesc<R> *__restrict__ d;
+    BatchCtl *b;
+    int ns, total, pshift;
+    __device__ __forceinline__ int take(int &scene) const {
+        const int i = atomicAdd(&b->next_p2g, 1);
+        if (i >= total) return -1;
+        scene = scene_of(b->pre_active, ns, i >> pshift);
+        return i - (b->pre_active[scene] << pshift);
     }
+    __device__ __forceinline__ const Params &params(int s) const { return d[s].P; }
+    __device__ __forceinline__ const Parts<R> &parts(int s) const { return d[s].A; }
+    __device__ __forceinline__ const int *active(int s) const { return d[s].active; }
+    __device__ __forceinline__ const int *start(int s) const { return d[s].start; }
+    __device__ __forceinline__ const int *cell_start(int s) const { return d[s].cell_start; }
+    __device__ __forceinline__ const int32_t *perm(int s) const { return d[s].perm; }
+    __device__ __forceinline__ long long *staging(int s) const { return d[s].staging; }
+    __device__ __forceinline__ const Ctl *ctl(int s) const { return d[s].ctl; }
+    __device__ __forceinline__ void fail(unsigned st) const { atomicOr(&d[0].ctl->status, st); }
+};
+template <class R, int ORD, bool THERM>
+__global__ void __launch_bounds__(P2GVar<R, ORD, 0>::THREADS, 1)
+    k_p2g_batch(const SceneDesc<R> *__restrict__ descs, BatchCtl *b, int nv, int pshift) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ P2GBuf bufs[2];
+    const int ns = b->nscenes;
+    const P2GBatchSrc<R> src{descs, b, ns, b->pre_active[ns] << pshift, pshift};
+    p2g_run<R, ORD, THERM>(src, smraw, bufs, nv, pshift);
 }
 
 template <class R, bool THERM>
@@ -4302,61 +3390,60 @@ void EXG_SFX(launch_state_reduce)(Ctx &c, unsigned long long *bounds, unsigned l
     EXG_CUDA_OK(cudaGetLastError());
 }
 
+// Threads and shared memory of a P2G block: as many warps as the shape has,
+// or as their records fit beside the two node blocks.
 template <class R, int ORD, bool TH>
-static void p2g_cell_t(Ctx &c, int flags) {
-    const int NCH = TH ? CH_ALL : CH_MOM_END;
-    const int B3 = c.P.B * c.P.B * c.P.B;
-    size_t sm = ((sizeof(SplineTables) + 15) & ~15) + sizeof(unsigned) * (fx_lo_words<R>() + 1) * NCH * B3;
-    auto kern = k_p2g_cell<R, ORD, TH>;
-    constexpr int nthr = P2GCfg<R, ORD, TH>::THREADS;
-    EXG_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    static int grid = 0;
-    static size_t gsm = 0;
-    if (!grid || gsm != sm) {
-        int dev = 0, nsm = 0, per = 0;
-        EXG_CUDA_OK(cudaGetDevice(&dev));
-        EXG_CUDA_OK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        EXG_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, nthr, sm));
-        grid = nsm * (per < 1 ? 1 : per);
-        gsm = sm;
-    }
-    kern<<<grid, nthr, sm, c.stream>>>(c.P, c.A<R>(), c.sb.active, c.sb.tile_start, c.sb.cell_start, c.sb.perm,
-                                       c.staging, c.ctl, flags);
-    EXG_CUDA_OK(cudaGetLastError());
+static int p2g_shape(int nv, int threads, size_t &sm) {
+    const size_t fixed = p2g_acc_off() + 2 * p2g_buf_bytes<R>(nv), per = p2g_warp_bytes<R, ORD, TH>();
+    const size_t most = 227 * 1024 - sizeof(P2GBuf) * 2 - 64;  // beside the static shared memory
+    if (fixed + per > most) throw std::runtime_error("P2G node block does not fit shared memory");
+    const int warps = std::min<int>(threads / 32, (int)((most - fixed) / per));
+    sm = fixed + per * warps;
+    return 32 * warps;
 }
 
-template <class R, int ORD, int V>
-static void p2g_fact_v(Ctx &c) {
-    const int B3 = c.P.B * c.P.B * c.P.B;
-    size_t sm = ((sizeof(SplineTables) + 15) & ~15) + sizeof(unsigned) * (fx_lo_words<R>() + 1) * CH_MOM_END * B3;
-    auto kern = k_p2g_fact<R, ORD, V>;
-    constexpr int nthr = P2GVar<R, ORD, V>::THREADS;
-    EXG_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    static int grid = 0;
-    static size_t gsm = 0;
-    if (!grid || gsm != sm) {
-        int dev = 0, nsm = 0, per = 0;
-        EXG_CUDA_OK(cudaGetDevice(&dev));
-        EXG_CUDA_OK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        EXG_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, nthr, sm));
-        grid = nsm * (per < 1 ? 1 : per);
-        gsm = sm;
+// Whether a block of (nearly) the default shape fits when tiles are split by
+// ps: FP32 cubic whole tiles leave room for 14 of its 16 warps, and the P2G
+// and nodal kernels together are no faster with half tiles (876 + 218 us
+// against 884 + 193 us on the 9 M-particle spheres).
+template <class R, int ORD>
+static bool p2g_fits_t(const Ctx &c, int ps) {
+    Params P = c.P;
+    P.Bz = (P.T >> ps) + P.hlo + P.hhi;
+    size_t sm;
+    constexpr int nthr = P2GVar<R, ORD, 0>::THREADS;
+    try {
+        return c.specs.use_temp ? p2g_shape<R, ORD, true>(p2g_values<true>(P), nthr, sm) * 8 >= nthr * 7
+                                : p2g_shape<R, ORD, false>(p2g_values<false>(P), nthr, sm) * 8 >= nthr * 7;
+    } catch (const std::exception &) {
+        return false;
     }
+}
+bool EXG_SFX(p2g_fits)(const Ctx &c, int ps) {
+    switch (c.P.uniform_order) {
+        case 1: return p2g_fits_t<EXG_R, 1>(c, ps);
+        case 2: return p2g_fits_t<EXG_R, 2>(c, ps);
+        default: return p2g_fits_t<EXG_R, 3>(c, ps);
+    }
+}
+
+template <class R, int ORD, bool TH, int V>
+static void p2g_v(Ctx &c) {
+    size_t sm;
+    const int nthr = p2g_shape<R, ORD, TH>(p2g_values<TH>(c.P), P2GVar<R, ORD, V>::THREADS, sm);
+    auto kern = k_p2g<R, ORD, TH, V>;
+    EXG_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    const int grid = persistent_grid(kern, sm, nthr);
     kern<<<grid, nthr, sm, c.stream>>>(c.P, c.A<R>(), c.sb.active, c.sb.tile_start, c.sb.cell_start, c.sb.perm,
                                        c.staging, c.ctl);
     EXG_CUDA_OK(cudaGetLastError());
 }
-
 template <class R, int ORD, bool TH>
-static void p2g_t(Ctx &c, int flags) {
-    if constexpr (P2GCfg<R, ORD, TH>::FACT) {
-        switch (c.p2g_var) {
-            case 1: p2g_fact_v<R, ORD, 1>(c); break;
-            case 2: p2g_fact_v<R, ORD, 2>(c); break;
-            default: p2g_fact_v<R, ORD, 0>(c); break;
-        }
-    } else {
-        p2g_cell_t<R, ORD, TH>(c, flags);
+static void p2g_t(Ctx &c) {
+    switch (c.p2g_var) {
+        case 1: p2g_v<R, ORD, TH, 1>(c); break;
+        case 2: p2g_v<R, ORD, TH, 2>(c); break;
+        default: p2g_v<R, ORD, TH, 0>(c); break;
     }
 }
 
@@ -4364,10 +3451,10 @@ void EXG_SFX(launch_p2g)(Ctx &c, int flags) {
     using R = EXG_R;
     const bool th = (flags & (PF_TEMP | PF_SRC)) != 0;
     switch (c.P.uniform_order) {
-        case 1: th ? p2g_t<R, 1, true>(c, flags) : p2g_t<R, 1, false>(c, flags); break;
-        case 2: th ? p2g_t<R, 2, true>(c, flags) : p2g_t<R, 2, false>(c, flags); break;
-        case 3: th ? p2g_t<R, 3, true>(c, flags) : p2g_t<R, 3, false>(c, flags); break;
-        default: th ? p2g_t<R, 0, true>(c, flags) : p2g_t<R, 0, false>(c, flags); break;
+        case 1: th ? p2g_t<R, 1, true>(c) : p2g_t<R, 1, false>(c); break;
+        case 2: th ? p2g_t<R, 2, true>(c) : p2g_t<R, 2, false>(c); break;
+        case 3: th ? p2g_t<R, 3, true>(c) : p2g_t<R, 3, false>(c); break;
+        default: th ? p2g_t<R, 0, true>(c) : p2g_t<R, 0, false>(c); break;
     }
 }
 
@@ -4702,19 +3789,14 @@ template <class R, int ORD>
 static void batch_p2g_t(Batch &b) {
     Ctx &c0 = *b.scenes[0];
     const SceneDesc<R> *d = reinterpret_cast<const SceneDesc<R> *>(b.desc[b.parity]);
-    const int B3 = c0.P.B * c0.P.B * c0.P.B;
-    constexpr int NCH = CH_MOM_END;
-    const size_t sm = ((sizeof(SplineTables) + 15) & ~15) + sizeof(unsigned) * (fx_lo_words<R>() + 1) * NCH * B3;
+    // scenes of a batch share the order, the tile and the split of their tiles
+    const int nv = p2g_values<false>(c0.P);
+    size_t sm;
+    const int nthr = p2g_shape<R, ORD, false>(nv, P2GVar<R, ORD, 0>::THREADS, sm);
     auto kern = k_p2g_batch<R, ORD, false>;
-    constexpr int nthr = P2GCfg<R, ORD, false>::THREADS;
     EXG_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    static int grid = 0;
-    static size_t gsm = 0;
-    if (!grid || gsm != sm) {
-        grid = persistent_grid(kern, sm, nthr);
-        gsm = sm;
-    }
-    kern<<<grid, nthr, sm, b.stream>>>(d, b.bctl, B3);
+    const int grid = persistent_grid(kern, sm, nthr);
+    kern<<<grid, nthr, sm, b.stream>>>(d, b.bctl, nv, c0.P.pshift);
     EXG_CUDA_OK(cudaGetLastError());
 }
 template <class R>
