@@ -46,11 +46,14 @@ bool fp64(const Ctx &c) { return c.precision == EXG_PREC_FP64; }
 // precision dispatch of the launchers
 #define DISPATCH(name, ...) (fp64(c) ? name##_fp64(__VA_ARGS__) : name##_fp32(__VA_ARGS__))
 
-// P2G items a launch should have at least: several for each block, so that the
-// last ones do not leave most of the GPU idle (a 15 thousand-particle dam
-// break's P2G 139 / 80 / 57 / 38 us with its tiles whole, in halves, quarters
-// and eighths)
-constexpr long long kP2GItems = 148 * 3;
+// Work items a launch should have at least: several for each block, so that the
+// last ones do not leave most of the GPU idle.  P2G: a 15 thousand-particle dam
+// break 139 / 80 / 57 / 38 us with its tiles whole, in halves, quarters and
+// eighths.  Fused G2P: the same scene 159 / 105 / 67 / 43 / 35 us with items of
+// 4096 / 2048 / 1024 / 512 / 256 particles, 540 thousand cubic particles 154 /
+// 159 / 115 / 109 / 117 us.  An item whose node block comes by plain loads
+// (periodic grids) costs more: 0.9 M particles 139 / 150 / 154 / 155 / 182 us.
+constexpr long long kP2GItems = 148 * 3, kG2PItems = 1000, kG2PItemsPlain = 148;
 
 template <class T>
 T *dalloc(size_t n) {
@@ -170,6 +173,7 @@ void build_params_for(const exg_specs &s, Params &P) {
     P.hhi = lin ? 1 : (P.dual ? 1 : 2);
     P.B = T + P.hlo + P.hhi;
     P.pshift = 0;
+    P.gshift = kG2PMaxShift;
     P.Bz = P.B;
     P.PS = P.B == 11 ? 130 : P.B * P.B;  // 130: 2 mod 32, the 4 x 4 columns of a cubic row on 16 banks
     for (int d = 0; d < 3; ++d)
@@ -323,30 +327,41 @@ void upload_parts(Ctx &c, const exg_particle_soa *h, const std::vector<int32_t> 
 
 void drop_graphs(Ctx &c);
 
-// Splits every tile into 1 << pshift P2G items for a launch over n particles
-// (of all scenes of a batch) and makes the staging array hold them.  An item is what one block takes at a time, so a
-// set of particles that fills fewer whole tiles than the GPU's blocks take at
-// once is split finer.
-void p2g_split(Ctx &c, long long n) {
+// Work split of the P2G and the fused G2P for launches over n particles (of all
+// scenes of a batch), np of them this scene's: a tile's P2G is cut into
+// 1 << pshift items, the fused G2P works on 1 << gshift particles at a time.
+// Makes the P2G's staging array hold its items.
+void p2g_split(Ctx &c, long long n, long long np) {
+    const bool f64 = fp64(c);
+    // staging words for a split: no more tiles hold particles than there are
+    // particles
+    auto words = [&](int ps) {
+        const long long nv = ((long long)c.nch * c.P.PS * ((c.P.T >> ps) + c.P.hlo + c.P.hhi) + 3) & ~3ll;
+        const long long tiles = std::min(c.P.ntiles, std::max(1ll, np)) << ps;
+        return (size_t)(tiles * (f64 ? stg_stride<double>(nv) : stg_stride<float>(nv)));
+    };
     int ps = 0;
     const long long tiles = std::max<long long>(1, n / (8ll * c.P.T * c.P.T * c.P.T));
     while (ps < c.P.tshift && (tiles << ps) < kP2GItems) ++ps;
+    // finer splits overlap more: at most twice the staging of whole tiles where
+    // that is more than 64 MB
+    while (ps > 0 && words(ps) > std::max(2 * words(0), (size_t)8 << 20)) --ps;
     // a block holds two node blocks and the records of its warps
     while (ps < c.P.tshift && !DISPATCH(p2g_fits, c, ps)) ++ps;
-    const int bz = (c.P.T >> ps) + c.P.hlo + c.P.hhi;
-    const long long nv = ((long long)c.nch * c.P.PS * bz + 3) & ~3ll;
-    const size_t need = (size_t)(c.P.ntiles << ps) * (fp64(c) ? stg_stride<double>(nv) : stg_stride<float>(nv));
-    if (need > c.staging_cap) {
+    if (words(ps) > c.staging_cap) {
         cudaFree(c.staging);
         c.staging = nullptr;
         c.staging_cap = 0;
-        c.staging = dalloc<long long>(need);
-        c.staging_cap = need;
+        c.staging = dalloc<long long>(words(ps));
+        c.staging_cap = words(ps);
         drop_graphs(c);
     }
-    if (ps != c.P.pshift || bz != c.P.Bz) drop_graphs(c);
+    int gs = kG2PMaxShift;
+    while (gs > kG2PMinShift && (n >> gs) < (c.tma ? kG2PItems : kG2PItemsPlain)) --gs;
+    if (ps != c.P.pshift || gs != c.P.gshift) drop_graphs(c);
+    c.P.gshift = gs;
     c.P.pshift = ps;
-    c.P.Bz = bz;
+    c.P.Bz = (c.P.T >> ps) + c.P.hlo + c.P.hhi;
 }
 
 }  // namespace
@@ -728,7 +743,6 @@ int exg_ctx_create(const exg_specs *specs, int device, exg_ctx **out) {
         EXG_CUDA_OK(cudaMemset(c.sb.touched_step, 0xff, sizeof(long long) * nt));  // -1: never
         EXG_CUDA_OK(cudaMemset(c.sb.slot, 0xff, sizeof(int) * nt));
         c.nch = specs->use_temp ? CH_ALL : CH_MOM_END;
-        p2g_split(c, 0);
         if (specs->use_temp) {
             // thermal wall pass: one entry per node of each non-periodic face
             c.n_tface = 0;
@@ -1000,7 +1014,7 @@ int exg_particles_upload(exg_ctx *ctx, const exg_particle_soa *p) {
         }
         EXG_CUDA_OK(cudaMemcpy(c.mat_dev, c.mats.data(), sizeof(Material) * c.mats.size(), cudaMemcpyHostToDevice));
         const bool temp = c.specs.use_temp != 0;
-        p2g_split(c, n);
+        p2g_split(c, n, n);
         if (g2p_lean(c) != lean_before) drop_graphs(c);  // the graphs hold the other G2P variant
         if (c.pa && n == c.np && n == c.cap) {
             // same particle count: the storage, sort buffers and step graphs stay
@@ -1889,7 +1903,7 @@ int exg_batch_step(exg_batch *B, int nsteps) {
             if (c->reduce_stale) do_reduce(*c);
         long long total = 0;
         for (Ctx *c : b.scenes) total += c->np;
-        for (Ctx *c : b.scenes) p2g_split(*c, total);  // one split for all: the launch covers every scene
+        for (Ctx *c : b.scenes) p2g_split(*c, total, c->np);  // one split for all: the launch covers every scene
         const bool changed = b.precision == EXG_PREC_FP64 ? batch_descriptors_fp64(b) : batch_descriptors_fp32(b);
         int lean = 1;
         for (Ctx *sc : b.scenes) lean = lean && g2p_lean(*sc);

@@ -59,16 +59,17 @@ struct Ctl {
     unsigned long long lost_fill;      // next slot for out-of-domain particles in the re-ordered storage
     int next_p2g;                      // dynamic tile counter of the P2G kernel (reset by k_scales)
     int next_g2p;                      // dynamic item counter of the fused G2P (reset by k_nodes)
-    int n_g2p_items;                   // work items of the fused G2P (chunks of kG2PChunk particles of a tile)
+    int n_g2p_items;                   // work items of the fused G2P
     int pad2;
 };
-// Particles of one work item of the fused G2P: a tile of more particles
-// (a pile-up) is split into several items, so that no item is much longer
-// than an ordinary tile.  Each item stages its tile's node block again, so
-// ordinary tiles (8 particles per cell of an 8^3 tile) stay whole: items of
-// 1024 made the 9 M-particle sphere step's G2P 5 % slower (FP64, whose node
-// block arrives single-buffered, 15 %).
-constexpr int kG2PChunk = 4096;
+// Particles of one work item of the fused G2P, as a power of two (the host
+// chooses it per particle count, g2p_chunk).  A tile of more particles (a
+// pile-up) is split into several items, so that no item is much longer than
+// an ordinary tile.  Each item stages its tile's node block again, so where
+// there are tiles enough for the GPU ordinary ones (8 particles per cell of an
+// 8^3 tile) stay whole: items of 1024 made the 9 M-particle sphere step's G2P
+// 5 % slower (FP64, whose node block arrives single-buffered, 15 %).
+constexpr int kG2PMaxShift = 12, kG2PMinShift = 8;
 
 // Per-tile stride of the P2G staging array, in 64-bit words, for nv
 // fixed-point values: FP32 state one 64-bit integer per value; FP64 state
@@ -125,6 +126,7 @@ struct Params {
     // words between z planes of a node block: B x B, padded where that spreads
     // the W x W columns a warp adds to over more shared-memory banks
     int PS;
+    int gshift;         // log2 of the particles of a fused-G2P work item
     double gravity[3];
     int external_loads;
     double slab_lo[3], slab_hi[3], extforce[3];

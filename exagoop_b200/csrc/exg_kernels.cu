@@ -199,16 +199,17 @@ __global__ void k_keys(Params P, double *x0, double *x1, double *x2, long long n
 
 // Exclusive scan of tile counts (one block, up to 32 warps): tile starts,
 // the ascending list of non-empty tiles, each tile's slot in it, and the
-// first fused-G2P work item of each active tile (ceil(count / kG2PChunk)
-// items a tile).  Each warp owns a contiguous chunk of tiles: it sums its
+// first fused-G2P work item of each active tile (ceil(count / chunk) items a
+// tile).  Each warp owns a contiguous chunk of tiles: it sums its
 // chunk in coalesced 32-tile steps, one barrier exchanges the warp totals,
 // and the warp walks its chunk again with warp-shuffle scans, writing
 // coalesced.  (A block-wide scan per 1024 tiles took 32 barrier-bound
 // rounds for 32,768 tiles; runs of tiles per thread made every store
 // uncoalesced.)
-__device__ __forceinline__ int tile_items(int c) { return (c + kG2PChunk - 1) / kG2PChunk; }
+// (chunk: a power of two, 1 << gsh)
+__device__ __forceinline__ int tile_items(int c, int gsh) { return (c + (1 << gsh) - 1) >> gsh; }
 __device__ __forceinline__ void tile_scan_block(int ntiles, const int *count, int *start, int *active, int *slot,
-                                                int *item_start, Ctl *ctl) {
+                                                int *item_start, Ctl *ctl, int gsh) {
     constexpr unsigned FULL = 0xffffffffu;
     __shared__ int s_tot[3][32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
@@ -219,7 +220,7 @@ __device__ __forceinline__ void tile_scan_block(int ntiles, const int *count, in
         const int c = count[i];
         tc += c;
         ta += c > 0;
-        ti += tile_items(c);
+        ti += tile_items(c, gsh);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -241,7 +242,7 @@ __device__ __forceinline__ void tile_scan_block(int ntiles, const int *count, in
     }
     for (int base = c0; base < c1; base += 32) {
         const int i = base + lane;
-        const int c = i < c1 ? count[i] : 0, a = c > 0, it = tile_items(c);
+        const int c = i < c1 ? count[i] : 0, a = c > 0, it = tile_items(c, gsh);
         int sc = c, sa = a, si = it;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -277,8 +278,8 @@ __device__ __forceinline__ void tile_scan_block(int ntiles, const int *count, in
     }
 }
 __global__ void k_tile_scan(int ntiles, const int *count, int *start, int *active, int *slot, int *item_start,
-                            Ctl *ctl) {
-    tile_scan_block(ntiles, count, start, active, slot, item_start, ctl);
+                            Ctl *ctl, int gsh) {
+    tile_scan_block(ntiles, count, start, active, slot, item_start, ctl, gsh);
 }
 
 // Tiles whose owned nodes the nodal kernel writes this step: tiles next to
@@ -678,6 +679,15 @@ struct Stc {
     static constexpr int W = (ORD == 1) ? 2 : 4;
     static constexpr int LO = (ORD == 1) ? 0 : -1;
 };
+
+// a[i] for a run-time i, in registers
+template <int W, class T>
+__device__ __forceinline__ T sel(const T (&a)[W], int i) {
+    T r = a[0];
+#pragma unroll
+    for (int k = 1; k < W; ++k) r = i == k ? a[k] : r;
+    return r;
+}
 
 // ---------------------------------------------------------------- K2 helpers
 // A node's fixed-point sum in shared memory.
@@ -1376,7 +1386,7 @@ template <class R>
 struct GlobalNodes {
     const R *v[3];
     const R *dv[3];
-    Params P;
+    const Params &P;
     __device__ __forceinline__ R get(int c, int i, int j, int k) const {
         long long n = node_index(P, i, j, k);
         if (n < 0) return R(0);
@@ -2277,7 +2287,7 @@ __global__ void __launch_bounds__(G2PVar<R, V>::THREADS, G2PVar<R, V>::MINB) k_g
     for (int c = 0; c < CH_ALL; ++c) run_b[c] = 0.0f;
     double run_speed = 0.0;  // largest CFL wave speed of the thread's particles
     bool red = false;
-    // work items (chunks of kG2PChunk particles of a tile) are taken in turn
+    // work items (chunks of 1 << P.gshift particles of a tile) are taken in turn
     // from a device counter (reset by k_nodes)
     const int nitems = ctl->n_g2p_items, nact = ctl->n_active_tiles;
     if (!use_tma) {
@@ -2291,10 +2301,10 @@ __global__ void __launch_bounds__(G2PVar<R, V>::THREADS, G2PVar<R, V>::MINB) k_g
             const int it = s_item;
             if (it >= nitems) break;
             const int w = s_w;
-            int kb = (w >= 0 && w < nact) ? (it - item_start[w]) * kG2PChunk : -1;
+            int kb = (w >= 0 && w < nact) ? (it - item_start[w]) << P.gshift : -1;
             if (kb < 0) status |= ST_BOUNDS;
             g2p_tile<R, ORD, LEAN>(tab, nb, P, A, Bo, Nd, bc, mats, active, start, count, perm, mode, w, dt, asr,
-                                   upd_vel, run_b, run_speed, red, status, false, kb, kb + kG2PChunk, np);
+                                   upd_vel, run_b, run_speed, red, status, false, kb, kb + (1 << P.gshift), np);
         }
     } else {
         // The node block of each tile comes by one TMA box from the nodal
@@ -2331,7 +2341,7 @@ __global__ void __launch_bounds__(G2PVar<R, V>::THREADS, G2PVar<R, V>::MINB) k_g
             const int it = s_items[cur];
             if (it >= nitems) break;
             const int w = s_ws[cur];
-            int kb = (w >= 0 && w < nact) ? (it - item_start[w]) * kG2PChunk : -1;
+            int kb = (w >= 0 && w < nact) ? (it - item_start[w]) << P.gshift : -1;
             if (kb < 0) status |= ST_BOUNDS;
             if (NBUF == 2 && threadIdx.x == 0) {
                 // the other buffer's last tile is done (the block synchronised)
@@ -2350,7 +2360,7 @@ __global__ void __launch_bounds__(G2PVar<R, V>::THREADS, G2PVar<R, V>::MINB) k_g
             }
             g2p_tile<R, ORD, LEAN>(tab, nb + cur * buf_words, P, A, Bo, Nd, bc, mats, active, start, count, perm,
                                    mode, w, dt, asr, upd_vel, run_b, run_speed, red, status, true, kb,
-                                   kb + kG2PChunk, np);
+                                   kb + (1 << P.gshift), np);
             if (NBUF == 2) {
                 cur ^= 1;
             } else {
@@ -2454,32 +2464,131 @@ __global__ void k_node_bcs(Params P, Nodes<R> Nd, NodeBCArgs bc, Ctl *ctl) {  //
     if (status) atomicOr(&ctl->status, status);
 }
 
+// The stencil of one particle for the gathers from the dense nodal arrays:
+// its weights (the nearest-node window for uniform quadratic) and, per axis,
+// the node offsets in elements, wrapped on periodic axes.  A node outside the
+// domain has weight 0 and is read at the nearest node of the domain, so the
+// loops over the window have neither tests nor modulo operations.  Weights
+// are formed in FP64 and rounded to R, as the tables' are.
 template <class R, int ORD>
-__global__ void __launch_bounds__(kThreads) k_g2p_simple(Params P, Parts<R> A, Nodes<R> Nd, long long np, int upd_vel,
-                                                         int upd_sr, double dt) {
+struct NodeGather {
+    static constexpr int W = ORD == 2 ? 3 : Stc<ORD>::W;
+    AxisW<R, W> a[3];
+    long long at[3][W];
+    __device__ __forceinline__ NodeGather(const SplineTables &tab, const Params &P, const double x[3], const int iv[3]) {
+        long long step = 1;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int nc = P.nc[d];
+            const bool per = P.periodic[d];
+            int base;
+            if constexpr (ORD == 2 || ORD == 3) {
+                const int c = ORD == 2 ? dual_bin(P, d, x[d]) : iv[d];
+                const double xw = ORD == 2 ? dual_x(P, d, x[d]) : x[d];
+                base = c - 1;
+                if (per || (c >= 3 && c <= nc - (ORD == 2 ? 3 : 4))) {
+                    AxisW<double, W> w;
+                    interior_weights<double, ORD>((xw - (P.plo[d] + c * P.dx[d])) * P.dxi[d], P.dxi[d], w);
+#pragma unroll
+                    for (int s = 0; s < W; ++s) {
+                        a[d].w[s] = (R)w.w[s];
+                        a[d].dw[s] = (R)w.dw[s];
+                    }
+                } else if constexpr (ORD == 2) {
+                    dual_axis_weights<R>(tab, P, d, xw, c, false, a[d]);
+                } else {
+                    axis_weights<R, W, -1>(tab, P, d, xw, c, a[d]);
+                }
+            } else {
+                axis_weights<R, W, Stc<ORD>::LO>(tab, P, d, x[d], iv[d], a[d]);
+                base = iv[d] + Stc<ORD>::LO;
+            }
+#pragma unroll
+            for (int s = 0; s < W; ++s) {
+                int i = base + s;
+                if (per)
+                    i = i < 0 ? i + nc : (i >= nc ? i - nc : i);
+                i = min(max(i, 0), nc);
+                at[d][s] = i * step;
+            }
+            step *= P.nn[d];
+        }
+    }
+};
+
+// G2P_Momentum on the dense nodal arrays, one thread per particle, the window
+// sum-factorized as in g2p_window.  Uniform orders; mixed per-axis orders take
+// g2p_particle.  With the direct form (FP64 tables for every weight, a modulo
+// index and a copy of the parameters per node) the gather of 140 thousand
+// cubic particles took 489 us, 31 us now.
+template <class R, int ORD>
+__global__ void __launch_bounds__(kThreads) k_g2p_simple(const __grid_constant__ Params P, Parts<R> A, Nodes<R> Nd,
+                                                         long long np, int upd_vel, int upd_sr, double dt) {
     __shared__ SplineTables tab;
     load_tables(&tab);
     __syncthreads();
     long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (p >= np || A.phase[p] != 0) return;
-    GlobalNodes<R> na;
-    for (int d = 0; d < 3; ++d) {
-        na.v[d] = Nd.c[EXG_N_VEL + d];
-        na.dv[d] = Nd.c[EXG_N_DVEL + d];
-    }
-    na.P = P;
     double x[3] = {A.x[0][p], A.x[1][p], A.x[2][p]};
     int iv[3];
     cell_of(P, x, iv);
     R v[3], vp[3], E[9], sr[6];
-    for (int d = 0; d < 3; ++d) {
-        v[d] = A.v[d][p];
-        vp[d] = A.vp[d][p];
-    }
-    for (int q = 0; q < 9; ++q) E[q] = A.E[q][p];
-    for (int c = 0; c < 6; ++c) sr[c] = A.sr[c][p];
+    for (int d = 0; d < 3; ++d) v[d] = vp[d] = R(0);
+    if (upd_vel)
+        for (int d = 0; d < 3; ++d) v[d] = A.v[d][p];
+    if (upd_sr)
+        for (int q = 0; q < 9; ++q) E[q] = A.E[q][p];
     double jf = 1.0;
-    g2p_particle<R, ORD>(tab, P, na, x, iv, upd_vel != 0, upd_sr != 0, v, vp, E, sr, dt, jf);
+    if constexpr (ORD == 0) {
+        const GlobalNodes<R> na{{Nd.c[EXG_N_VEL], Nd.c[EXG_N_VEL + 1], Nd.c[EXG_N_VEL + 2]},
+                                {Nd.c[EXG_N_DVEL], Nd.c[EXG_N_DVEL + 1], Nd.c[EXG_N_DVEL + 2]},
+                                P};
+        g2p_particle<R, ORD>(tab, P, na, x, iv, upd_vel != 0, upd_sr != 0, v, vp, E, sr, dt, jf);
+    } else {
+        const NodeGather<R, ORD> g(tab, P, x, iv);
+        constexpr int W = NodeGather<R, ORD>::W;
+        R V[3] = {R(0), R(0), R(0)}, D[3] = {R(0), R(0), R(0)};
+        R G[3][3] = {{R(0), R(0), R(0)}, {R(0), R(0), R(0)}, {R(0), R(0), R(0)}};
+#pragma unroll 1
+        for (int sz = 0; sz < W; ++sz) {
+            R Sv[3] = {R(0), R(0), R(0)}, Sd[3] = {R(0), R(0), R(0)}, Sy[3] = {R(0), R(0), R(0)},
+              Sx[3] = {R(0), R(0), R(0)};
+            const R wz = sel<W>(g.a[2].w, sz), dwz = sel<W>(g.a[2].dw, sz);
+            const long long az = sel<W>(g.at[2], sz);
+#pragma unroll
+            for (int sy = 0; sy < W; ++sy) {
+                const long long row = az + g.at[1][sy];
+                R a[3] = {R(0), R(0), R(0)}, bx[3] = {R(0), R(0), R(0)}, c[3] = {R(0), R(0), R(0)};
+#pragma unroll
+                for (int sx = 0; sx < W; ++sx) {
+                    const long long q = row + g.at[0][sx];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        const R nv = Nd.c[EXG_N_VEL + d][q];
+                        a[d] = fma(g.a[0].w[sx], nv, a[d]);
+                        bx[d] = fma(g.a[0].dw[sx], nv, bx[d]);
+                        if (upd_vel) c[d] = fma(g.a[0].w[sx], Nd.c[EXG_N_DVEL + d][q], c[d]);
+                    }
+                }
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    Sv[d] = fma(g.a[1].w[sy], a[d], Sv[d]);
+                    Sd[d] = fma(g.a[1].w[sy], c[d], Sd[d]);
+                    Sy[d] = fma(g.a[1].dw[sy], a[d], Sy[d]);
+                    Sx[d] = fma(g.a[1].w[sy], bx[d], Sx[d]);
+                }
+            }
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                V[d] = fma(wz, Sv[d], V[d]);
+                D[d] = fma(wz, Sd[d], D[d]);
+                G[d][0] = fma(wz, Sx[d], G[d][0]);
+                G[d][1] = fma(wz, Sy[d], G[d][1]);
+                G[d][2] = fma(dwz, Sv[d], G[d][2]);
+            }
+        }
+        g2p_finish<R>(P, upd_vel != 0, upd_sr != 0, V, D, G, v, vp, E, sr, dt, jf);
+    }
     if (sizeof(R) == 4 && upd_sr) A.J[p] *= jf;  // FP32 state: J kept in FP64 alongside F
     if (upd_vel)
         for (int d = 0; d < 3; ++d) {
@@ -2844,8 +2953,8 @@ __global__ void k_temp_levelset(Params P, Nodes<R> Nd, const double *phi, int b,
 // T += interpolated nodal temperature increment (scheme of the x order, as
 // the reference selects it) and q = -k grad T from the nodal temperatures.
 template <class R, int ORD>
-__global__ void __launch_bounds__(kThreads) k_g2p_temp(Params P, Parts<R> A, Nodes<R> Nd, long long np, int upd_T,
-                                                       int upd_q) {
+__global__ void __launch_bounds__(kThreads) k_g2p_temp(const __grid_constant__ Params P, Parts<R> A, Nodes<R> Nd,
+                                                       long long np, int upd_T, int upd_q) {
     __shared__ SplineTables tab;
     load_tables(&tab);
     __syncthreads();
@@ -2854,8 +2963,49 @@ __global__ void __launch_bounds__(kThreads) k_g2p_temp(Params P, Parts<R> A, Nod
     const double x[3] = {A.x[0][p], A.x[1][p], A.x[2][p]};
     int iv[3];
     cell_of(P, x, iv);
+    const R *Tn = Nd.c[EXG_N_TEMPERATURE], *dT = Nd.c[EXG_N_DELTA_TEMPERATURE];
+    if constexpr (ORD != 0) {
+        // both gathers over one window, sum-factorized (the two windows of 64
+        // cells each with a test and a modulo index per node took 684 us on
+        // the 1.6 M-particle column, 72 us now)
+        const NodeGather<R, ORD> g(tab, P, x, iv);
+        constexpr int W = NodeGather<R, ORD>::W;
+        R dt = R(0), gr[3] = {R(0), R(0), R(0)};
+#pragma unroll
+        for (int sz = 0; sz < W; ++sz) {
+            R Sd = R(0), Sv = R(0), Sx = R(0), Sy = R(0);
+#pragma unroll
+            for (int sy = 0; sy < W; ++sy) {
+                const long long row = g.at[2][sz] + g.at[1][sy];
+                R a = R(0), b = R(0), c = R(0);
+#pragma unroll
+                for (int sx = 0; sx < W; ++sx) {
+                    const long long q = row + g.at[0][sx];
+                    if (upd_q) {
+                        const R t = Tn[q];
+                        a = fma(g.a[0].w[sx], t, a);
+                        b = fma(g.a[0].dw[sx], t, b);
+                    }
+                    if (upd_T) c = fma(g.a[0].w[sx], dT[q], c);
+                }
+                Sv = fma(g.a[1].w[sy], a, Sv);
+                Sy = fma(g.a[1].dw[sy], a, Sy);
+                Sx = fma(g.a[1].w[sy], b, Sx);
+                Sd = fma(g.a[1].w[sy], c, Sd);
+            }
+            dt = fma(g.a[2].w[sz], Sd, dt);
+            gr[0] = fma(g.a[2].w[sz], Sx, gr[0]);
+            gr[1] = fma(g.a[2].w[sz], Sy, gr[1]);
+            gr[2] = fma(g.a[2].dw[sz], Sv, gr[2]);
+        }
+        if (upd_T) A.T[p] = A.T[p] + (double)dt;
+        if (upd_q) {
+            const R k = A.kc[p];
+            for (int d = 0; d < 3; ++d) A.q[d][p] = -k * gr[d];
+        }
+        return;
+    }
     if (upd_T) {
-        const R *dT = Nd.c[EXG_N_DELTA_TEMPERATURE];
         R wx[4], wy[4], wz[4];
         interp_axis<R>(tab, P, P.order[0], 0, x[0], iv[0], wx);
         interp_axis<R>(tab, P, P.order[0], 1, x[1], iv[1], wy);
@@ -2873,7 +3023,6 @@ __global__ void __launch_bounds__(kThreads) k_g2p_temp(Params P, Parts<R> A, Nod
     }
     if (upd_q) {
         constexpr int W = Stc<ORD>::W, LO = Stc<ORD>::LO;
-        const R *Tn = Nd.c[EXG_N_TEMPERATURE];
         AxisW<R, W> ax, ay, az;
         axis_weights<R, W, LO>(tab, P, 0, x[0], iv[0], ax);
         axis_weights<R, W, LO>(tab, P, 1, x[1], iv[1], ay);
@@ -3073,7 +3222,7 @@ __global__ void __launch_bounds__(kBatchThreads) k_bb_keys(const SortDesc *__res
 
 __global__ void k_bb_tile_scan(const SortDesc *__restrict__ d) {
     const SortDesc &x = d[blockIdx.x];
-    tile_scan_block((int)x.P.ntiles, x.tile_count, x.tile_start, x.active, x.slot, x.item_start, x.ctl);
+    tile_scan_block((int)x.P.ntiles, x.tile_count, x.tile_start, x.active, x.slot, x.item_start, x.ctl, x.P.gshift);
 }
 
 __global__ void __launch_bounds__(kBatchThreads) k_bb_scatter(const SortDesc *__restrict__ d,
@@ -3335,7 +3484,7 @@ void launch_keys(Ctx &c) {
 
 void launch_sort_rest(Ctx &c, bool touched_list) {
     k_tile_scan<<<1, 1024, 0, c.stream>>>((int)c.P.ntiles, c.sb.tile_count, c.sb.tile_start, c.sb.active, c.sb.slot,
-                                          c.sb.item_start, c.ctl);
+                                          c.sb.item_start, c.ctl, c.P.gshift);
     if (c.np > 0)
         k_scatter<<<nblocks(c.np), kThreads, 0, c.stream>>>(c.np, c.sb.key, 3 * c.P.tshift, c.sb.tile_start,
                                                             c.sb.tile_fill, c.sb.bucket);
