@@ -1148,22 +1148,32 @@ __device__ __forceinline__ void write_rec(R *rec, long long ni, const double v[3
 }
 
 // ---------------------------------------------------------------- K3 nodes
-// One CTA per tile; each thread owns nodes of the tile, adds the fixed-point
-// partials of the <= 8 node blocks covering the node (exact integer sums),
-// converts to FP64 and applies the nodal operations of the mode.
-// One tile of the nodal kernel: every owned node of tile tiles[w] (or w).
+// Each thread owns a node of a tile, adds the fixed-point partials of the node
+// blocks covering it (exact integer sums), converts to FP64 and applies the
+// nodal operations of the mode.  A block of 128 threads takes a quarter of an
+// 8^3 tile: the kernel is a chain of dependent loads per node, so a small
+// scene's few tiles are spread over four times the SMs and no thread walks two
+// nodes (against 256 threads a tile: 15 thousand particles 28 -> 18 us, 540
+// thousand 48 -> 33, 9 M 217 -> 193).
+// Part `part` of tile tiles[w] (or w).
+constexpr int kNodesThreads = 128;
+__host__ __device__ __forceinline__ int nodes_parts(const Params &P) {
+    return max(1, P.T * P.T * P.T / kNodesThreads);
+}
 template <class R, bool THERM, bool LEAN = false>
 __device__ __forceinline__ void nodes_tile(const Params &P, const Nodes<R> &Nd, const NodeBCArgs &bc, const int *tiles,
                                            const int *slot, const long long *staging, const double *isc, double dt,
-                                           int mode, int flags, int w, unsigned &status) {
+                                           int mode, int flags, int w, int part, unsigned &status) {
     constexpr int NCH = THERM ? CH_ALL : CH_MOM_END;
     const int B = P.B, T = P.T;
     const int zs = P.tshift - P.pshift, parts = 1 << P.pshift;  // log2 of an item's z planes, items per tile
     const int t = tiles ? tiles[w] : w;
     int tc[3];
     tile_coords(P, t, tc);
-    for (int ln = threadIdx.x; ln < T * T * T; ln += blockDim.x) {
-        const int l[3] = {ln % T, (ln / T) % T, ln / (T * T)};
+    {
+        const int ln = part * kNodesThreads + (int)threadIdx.x;
+        if (ln >= T * T * T) return;
+        const int l[3] = {ln & (T - 1), (ln >> P.tshift) & (T - 1), ln >> (2 * P.tshift)};
         int nid[3];
         bool ok = true;
         for (int d = 0; d < 3; ++d) {
@@ -1171,7 +1181,7 @@ __device__ __forceinline__ void nodes_tile(const Params &P, const Nodes<R> &Nd, 
             const int nown = P.periodic[d] ? P.nc[d] : P.nc[d] + 1;
             ok = ok && nid[d] < nown;
         }
-        if (!ok) continue;
+        if (!ok) return;
         FxSum<R> accv[NCH];
 #pragma unroll
         for (int c = 0; c < NCH; ++c) accv[c] = FxSum<R>();
@@ -1340,16 +1350,13 @@ __device__ __forceinline__ void nodes_tile(const Params &P, const Nodes<R> &Nd, 
     }
 }
 
-// Four 256-thread blocks per SM (64 registers, some spilled): the per-node
-// work is a chain of dependent loads (slot, then up to eight staging
-// blocks), so occupancy decides its speed (the dam break's nodal update
-// 0.171 ms with one block per SM and no register cap, 0.108 / 0.086 / 0.080
-// ms with two / three / four blocks)
-#ifndef EXG_NODES_MINB
-#define EXG_NODES_MINB 4
-#endif
+// 32 warps per SM (64 registers, some spilled): the per-node work is a chain of
+// dependent loads (slot, then the staging blocks), so occupancy decides its
+// speed (the dam break's nodal update 0.171 ms with 8 warps per SM and no
+// register cap, 0.108 / 0.086 / 0.080 ms with 16 / 24 / 32)
+constexpr int kNodesMinB = 8;
 template <class R, bool THERM, bool LEAN = false>
-__global__ void __launch_bounds__(kThreads, EXG_NODES_MINB) k_nodes(Params P, Nodes<R> Nd, NodeBCArgs bc, const int *tiles,
+__global__ void __launch_bounds__(kNodesThreads, kNodesMinB) k_nodes(Params P, Nodes<R> Nd, NodeBCArgs bc, const int *tiles,
                                                     const int *slot, const long long *staging, Ctl *ctl, int mode,
                                                     int flags) {
     constexpr int NCH = THERM ? CH_ALL : CH_MOM_END;
@@ -1361,9 +1368,9 @@ __global__ void __launch_bounds__(kThreads, EXG_NODES_MINB) k_nodes(Params P, No
     // the fused G2P that follows takes its tiles from 0 (it starts after
     // this kernel ends, and the previous one has ended)
     if (blockIdx.x == 0 && threadIdx.x == 0) ctl->next_g2p = 0;
-    const int nitems = tiles ? ctl->n_touched_tiles : (int)P.ntiles;
+    const int np = nodes_parts(P), nitems = (tiles ? ctl->n_touched_tiles : (int)P.ntiles) * np;
     for (int w = blockIdx.x; w < nitems; w += gridDim.x)
-        nodes_tile<R, THERM, LEAN>(P, Nd, bc, tiles, slot, staging, isc, dt, mode, flags, w, status);
+        nodes_tile<R, THERM, LEAN>(P, Nd, bc, tiles, slot, staging, isc, dt, mode, flags, w / np, w % np, status);
     if (status) atomicOr(&ctl->status, status);
 }
 
@@ -3328,11 +3335,11 @@ __global__ void __launch_bounds__(P2GVar<R, ORD, 0>::THREADS, 1)
 }
 
 template <class R, bool THERM>
-__global__ void __launch_bounds__(kThreads, EXG_NODES_MINB) k_nodes_batch(const SceneDesc<R> *__restrict__ descs, BatchCtl *b, int mode,
+__global__ void __launch_bounds__(kNodesThreads, kNodesMinB) k_nodes_batch(const SceneDesc<R> *__restrict__ descs, BatchCtl *b, int mode,
                                                           int flags) {
     constexpr int NCH = THERM ? CH_ALL : CH_MOM_END;
     __shared__ int s_item, s_scene;
-    const int ns = b->nscenes, total = b->pre_touched[ns];
+    const int ns = b->nscenes, np = nodes_parts(descs[0].P), total = b->pre_touched[ns];
     int cur = -1;
     unsigned status = 0;
     double isc[NCH], dt = 0.0;
@@ -3354,8 +3361,9 @@ __global__ void __launch_bounds__(kThreads, EXG_NODES_MINB) k_nodes_batch(const 
             for (int c = 0; c < NCH; ++c) isc[c] = sd.ctl->inv_scale[c];
             dt = sd.ctl->dt;
         }
-        nodes_tile<R, THERM>(sd.P, sd.N, sd.bc, sd.touched, sd.slot, sd.staging, isc, dt, mode, flags,
-                             i - b->pre_touched[s], status);
+        for (int part = 0; part < np; ++part)
+            nodes_tile<R, THERM>(sd.P, sd.N, sd.bc, sd.touched, sd.slot, sd.staging, isc, dt, mode, flags,
+                                 i - b->pre_touched[s], part, status);
         __syncthreads();
     }
     if (cur >= 0 && status) atomicOr(&descs[cur].ctl->status, status);
@@ -3617,20 +3625,20 @@ void EXG_SFX(launch_nodes)(Ctx &c, int mode, int flags, bool all_tiles) {
     for (int h = 0; h < 2; ++h)
         for (int d = 0; d < 3; ++d) lean = lean && bc.udf[h][d] == nullptr;
     static int pgrid = 0, pgrid_th = 0, pgrid_lean = 0;
-    if (!pgrid) pgrid = persistent_grid(k_nodes<R, false>, 0);
-    if (!pgrid_th) pgrid_th = persistent_grid(k_nodes<R, true>, 0);
-    if (!pgrid_lean) pgrid_lean = persistent_grid(k_nodes<R, false, true>, 0);
+    if (!pgrid) pgrid = persistent_grid(k_nodes<R, false>, 0, kNodesThreads);
+    if (!pgrid_th) pgrid_th = persistent_grid(k_nodes<R, true>, 0, kNodesThreads);
+    if (!pgrid_lean) pgrid_lean = persistent_grid(k_nodes<R, false, true>, 0, kNodesThreads);
     const int pg = th ? pgrid_th : (lean ? pgrid_lean : pgrid);  // the grid of the variant launched
-    int grid = all_tiles ? (int)std::min<long long>(c.P.ntiles, pg) : pg;
+    int grid = (int)std::min<long long>(c.P.ntiles * nodes_parts(c.P), pg);
     const int *tiles = all_tiles ? nullptr : c.sb.touched;
     if (th)
-        k_nodes<R, true><<<grid, kThreads, 0, c.stream>>>(c.P, c.N<R>(), bc, tiles, c.sb.slot, c.staging, c.ctl, mode,
+        k_nodes<R, true><<<grid, kNodesThreads, 0, c.stream>>>(c.P, c.N<R>(), bc, tiles, c.sb.slot, c.staging, c.ctl, mode,
                                                           flags);
     else if (lean)
-        k_nodes<R, false, true><<<grid, kThreads, 0, c.stream>>>(c.P, c.N<R>(), bc, tiles, c.sb.slot, c.staging,
+        k_nodes<R, false, true><<<grid, kNodesThreads, 0, c.stream>>>(c.P, c.N<R>(), bc, tiles, c.sb.slot, c.staging,
                                                                  c.ctl, mode, flags);
     else
-        k_nodes<R, false><<<grid, kThreads, 0, c.stream>>>(c.P, c.N<R>(), bc, tiles, c.sb.slot, c.staging, c.ctl,
+        k_nodes<R, false><<<grid, kNodesThreads, 0, c.stream>>>(c.P, c.N<R>(), bc, tiles, c.sb.slot, c.staging, c.ctl,
                                                            mode, flags);
     EXG_CUDA_OK(cudaGetLastError());
 }
@@ -3952,8 +3960,8 @@ template <class R>
 static void batch_nodes_t(Batch &b) {
     const SceneDesc<R> *d = reinterpret_cast<const SceneDesc<R> *>(b.desc[b.parity]);
     static int grid = 0;
-    if (!grid) grid = persistent_grid(k_nodes_batch<R, false>, 0);
-    k_nodes_batch<R, false><<<grid, kThreads, 0, b.stream>>>(d, b.bctl, NM_FUSED, PF_MASS | PF_VEL | PF_FORCE);
+    if (!grid) grid = persistent_grid(k_nodes_batch<R, false>, 0, kNodesThreads);
+    k_nodes_batch<R, false><<<grid, kNodesThreads, 0, b.stream>>>(d, b.bctl, NM_FUSED, PF_MASS | PF_VEL | PF_FORCE);
     EXG_CUDA_OK(cudaGetLastError());
 }
 template <class R, int ORD>
