@@ -565,8 +565,8 @@ int status_from_ctl(Ctx &c) {
 
 // Sort by cell key for the current storage order (Redistribute).
 void do_sort(Ctx &c, bool touched) {
-    launch_keys(c);
-    launch_sort_rest(c, touched);
+    launch_keys(c, true);
+    launch_sort_rest(c, touched, nullptr);
     c.parts_sorted = true;
 }
 
@@ -579,16 +579,13 @@ void do_reduce(Ctx &c) {
 
 // One fused step, enqueued on c.stream (capturable).
 void enqueue_step(Ctx &c) {
-    EXG_CUDA_OK(cudaMemcpyAsync(c.bounds_cur, &c.ctl->bound_bits[0], sizeof(unsigned long long) * CH_ALL,
-                                cudaMemcpyDeviceToDevice, c.stream));
-    launch_dt_finalize(c, true);
+    launch_step_start(c);
     if (c.timing) EXG_CUDA_OK(cudaEventRecord(c.ev[0], c.stream));
     nvtxRangePushA("step: sort (Redistribute)");
-    launch_keys(c);
-    launch_sort_rest(c, true);
+    launch_keys(c, false);
+    launch_sort_rest(c, true, c.bounds_cur);
     nvtxRangePop();
     if (c.timing) EXG_CUDA_OK(cudaEventRecord(c.ev[1], c.stream));
-    launch_scales_from(c, c.bounds_cur);
     const bool th = c.specs.use_temp != 0;
     const bool musl = c.specs.stress_update_scheme != 0;
     const int tflags = th ? (PF_TEMP | PF_SRC) : 0;
@@ -622,9 +619,8 @@ void enqueue_step(Ctx &c) {
         }
         DISPATCH(launch_g2p_fused, c, GM_STRAIN);
     }
-    DISPATCH(launch_copy_lost, c);
+    DISPATCH(launch_step_end, c);
     if (c.timing) EXG_CUDA_OK(cudaEventRecord(c.ev[4], c.stream));
-    launch_time_advance(c);
 }
 
 void swap_parts(Ctx &c) {

@@ -77,12 +77,14 @@ void d2h_int(Ctx &c, const void *src, int bytes, const int32_t *pid, int32_t *ho
 // precision builds of that file)
 void upload_tables_fp64();
 void upload_tables_fp32();
-void launch_keys(Ctx &c);
-void launch_sort_rest(Ctx &c, bool touched_list);
+void launch_step_start(Ctx &c);
+void launch_keys(Ctx &c, bool zero_counts);
+// touched_list: also the list of tiles the nodal kernel writes and, from
+// bounds when given, the P2G's fixed-point scales
+void launch_sort_rest(Ctx &c, bool touched_list, const unsigned long long *bounds);
 void launch_dt_finalize(Ctx &c, bool reset);
 void launch_reset_accum(Ctx &c, unsigned long long *bounds, unsigned long long *dtmin);
 void launch_scales_from(Ctx &c, const unsigned long long *bounds);
-void launch_time_advance(Ctx &c);
 void launch_node_reset(Ctx &c);
 #define EXG_DECL_PREC(sfx)                                                      \
     void launch_state_reduce##sfx(Ctx &c, unsigned long long *bounds, unsigned long long *dtmin); \
@@ -90,7 +92,7 @@ void launch_node_reset(Ctx &c);
     void launch_p2g##sfx(Ctx &c, int flags);                                     \
     void launch_nodes##sfx(Ctx &c, int mode, int flags, bool all_tiles);         \
     void launch_g2p_fused##sfx(Ctx &c, int mode);                                \
-    void launch_copy_lost##sfx(Ctx &c);                                          \
+    void launch_step_end##sfx(Ctx &c);                                           \
     void launch_g2p_simple##sfx(Ctx &c, int uv, int us, double dt);              \
     void launch_node_backup##sfx(Ctx &c);                                        \
     void launch_node_time_update##sfx(Ctx &c, double dt);                        \

@@ -291,22 +291,27 @@ __device__ __forceinline__ void touched_body(const Params &P, const int *count, 
     if (t >= P.ntiles) return;
     int tc[3];
     tile_coords(P, t, tc);
-    bool now = false;
-    for (int dz = -1; dz <= 1 && !now; ++dz)
-        for (int dy = -1; dy <= 1 && !now; ++dy)
-            for (int dx = -1; dx <= 1 && !now; ++dx) {
+    // all 27 counts are loaded together: stopping at the first non-empty tile
+    // made each load wait for the one before
+    int any = 0;
+#pragma unroll
+    for (int dz = -1; dz <= 1; ++dz)
+#pragma unroll
+        for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+            for (int dx = -1; dx <= 1; ++dx) {
                 int s[3] = {tc[0] + dx, tc[1] + dy, tc[2] + dz};
                 bool ok = true;
+#pragma unroll
                 for (int d = 0; d < 3; ++d) {
                     if (s[d] < 0 || s[d] >= P.ntile[d]) {
-                        if (P.periodic[d])
-                            s[d] = (s[d] + P.ntile[d]) % P.ntile[d];
-                        else
-                            ok = false;
+                        ok = ok && P.periodic[d];
+                        s[d] += s[d] < 0 ? P.ntile[d] : -P.ntile[d];
                     }
                 }
-                if (ok && count[(s[2] * P.ntile[1] + s[1]) * P.ntile[0] + s[0]] > 0) now = true;
+                any |= ok ? count[(s[2] * P.ntile[1] + s[1]) * P.ntile[0] + s[0]] : 0;
             }
+    const bool now = any > 0;
     long long cur = ctl->steps;
     long long prev = touched_step[t];
     if (now || prev == cur - 1) {
@@ -315,7 +320,13 @@ __device__ __forceinline__ void touched_body(const Params &P, const int *count, 
     }
     if (now) touched_step[t] = cur;
 }
-__global__ void k_touched(Params P, const int *count, int *touched, long long *touched_step, Ctl *ctl) {
+// With bounds, block 0 also forms the P2G's fixed-point scales (the tile sort,
+// which finds the largest cell, has ended), a launch less per step.
+__device__ __forceinline__ void scales_body(Ctl *ctl, int stencil_cells, int bits, const unsigned long long *bounds,
+                                            int c);
+__global__ void k_touched(const __grid_constant__ Params P, const int *count, int *touched, long long *touched_step,
+                          Ctl *ctl, int stencil_cells, int bits, const unsigned long long *bounds) {
+    if (bounds && blockIdx.x == 0 && threadIdx.x < 32) scales_body(ctl, stencil_cells, bits, bounds, threadIdx.x);
     touched_body(P, count, touched, touched_step, ctl, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -474,7 +485,7 @@ __device__ __forceinline__ void tile_sort_item(int *sm, const int *active, const
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kThreads) k_tile_sort(const int *active, const int *start, const int *count,
+__global__ void __launch_bounds__(1024) k_tile_sort(const int *active, const int *start, const int *count,
                                                         const uint32_t *key, const int32_t *bucket, int32_t *scratch,
                                                         int32_t *perm, int *cell_start, int ncell, Ctl *ctl) {
     extern __shared__ int sm[];
@@ -507,6 +518,21 @@ __device__ __forceinline__ void dt_finalize_body(const Params &P, Ctl *ctl, int 
 }
 __global__ void k_dt_finalize(Params P, Ctl *ctl, int reset) { dt_finalize_body(P, ctl, reset); }
 
+// Start of a fused step in one launch: the step's P2G bounds (those of the
+// last G2P), dt and the accumulator reset, zeroed tile counts.
+__global__ void k_step_start(const __grid_constant__ Params P, Ctl *ctl, unsigned long long *bounds_cur, int *tile_count,
+                             int *tile_fill) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i == 0) {
+        for (int c = 0; c < CH_ALL; ++c) bounds_cur[c] = ctl->bound_bits[c];
+        dt_finalize_body(P, ctl, 1);
+    }
+    if (i < P.ntiles) {
+        tile_count[i] = 0;
+        tile_fill[i] = 0;
+    }
+}
+
 // Fixed-point scales: a channel's node sum is bounded by
 // (particles per cell) x (stencil cells) x (largest per-particle term);
 // the scale 2^e keeps twice that bound below 2^bits (see fx_add_r).
@@ -530,11 +556,6 @@ __device__ __forceinline__ void scales_body(Ctl *ctl, int stencil_cells, int bit
 }
 __global__ void k_scales(Ctl *ctl, int stencil_cells, int bits, const unsigned long long *bounds) {
     scales_body(ctl, stencil_cells, bits, bounds, threadIdx.x);
-}
-
-__global__ void k_time_advance(Ctl *ctl) {
-    ctl->time += ctl->dt;
-    ctl->steps += 1;
 }
 
 #endif  // EXG_R_FP64
@@ -2423,13 +2444,22 @@ __device__ __forceinline__ void copy_particle(const Parts<R> &A, long long i, Pa
     }
 }
 
+// End of a fused step: the time advance, and the lost particles.  Usually there
+// are none and no key is read, so the launch has only enough blocks to copy
+// quickly when there are (one block per 256 particles spent 18 us on 8 M
+// particles finding that out).
 template <class R>
-__global__ void k_copy_lost(Parts<R> A, Parts<R> Bo, const uint32_t *key, long long np, Ctl *ctl, int temp) {
-    if (ctl->lost == 0) return;  // the usual case: nothing to copy, no key to read
-    long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= np || key[i] != 0xFFFFFFFFu) return;
-    long long j = ctl->n_sorted + (long long)atomicAdd(&ctl->lost_fill, 1ull);
-    copy_particle<R>(A, i, Bo, j, temp != 0);
+__global__ void k_step_end(Parts<R> A, Parts<R> Bo, const uint32_t *key, long long np, Ctl *ctl, int temp) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        ctl->time += ctl->dt;
+        ctl->steps += 1;
+    }
+    if (ctl->lost == 0) return;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < np; i += (long long)gridDim.x * blockDim.x) {
+        if (key[i] != 0xFFFFFFFFu) continue;
+        const long long j = ctl->n_sorted + (long long)atomicAdd(&ctl->lost_fill, 1ull);
+        copy_particle<R>(A, i, Bo, j, temp != 0);
+    }
 }
 
 // ---------------------------------------------------------------- unfused L5 kernels
@@ -3480,9 +3510,23 @@ static NodeBCArgs make_bc(Ctx &c) {
 }
 
 #if defined(EXG_R_FP64)
-void launch_keys(Ctx &c) {
-    EXG_CUDA_OK(cudaMemsetAsync(c.sb.tile_count, 0, sizeof(int) * c.P.ntiles, c.stream));
-    EXG_CUDA_OK(cudaMemsetAsync(c.sb.tile_fill, 0, sizeof(int) * c.P.ntiles, c.stream));
+static int stencil_cells(const Ctx &c) {
+    const int W = (c.P.uniform_order == 1) ? 2 : (c.P.dual ? 3 : 4);
+    return W * W * W;
+}
+static int scale_bits(const Ctx &c) { return c.precision == EXG_PREC_FP64 ? kFxBits64 : kFxBits32; }
+
+void launch_step_start(Ctx &c) {
+    k_step_start<<<nblocks(c.P.ntiles), kThreads, 0, c.stream>>>(c.P, c.ctl, c.bounds_cur, c.sb.tile_count,
+                                                                 c.sb.tile_fill);
+    EXG_CUDA_OK(cudaGetLastError());
+}
+
+void launch_keys(Ctx &c, bool zero_counts) {
+    if (zero_counts) {
+        EXG_CUDA_OK(cudaMemsetAsync(c.sb.tile_count, 0, sizeof(int) * c.P.ntiles, c.stream));
+        EXG_CUDA_OK(cudaMemsetAsync(c.sb.tile_fill, 0, sizeof(int) * c.P.ntiles, c.stream));
+    }
     double **x = c.precision == EXG_PREC_FP64 ? c.A<double>().x : c.A<float>().x;
     if (c.np > 0)
         k_keys<<<nblocks(c.np), kThreads, 0, c.stream>>>(c.P, x[0], x[1], x[2], c.np, c.sb.key, c.sb.tile_count, c.ctl,
@@ -3490,7 +3534,7 @@ void launch_keys(Ctx &c) {
     EXG_CUDA_OK(cudaGetLastError());
 }
 
-void launch_sort_rest(Ctx &c, bool touched_list) {
+void launch_sort_rest(Ctx &c, bool touched_list, const unsigned long long *bounds) {
     k_tile_scan<<<1, 1024, 0, c.stream>>>((int)c.P.ntiles, c.sb.tile_count, c.sb.tile_start, c.sb.active, c.sb.slot,
                                           c.sb.item_start, c.ctl, c.P.gshift);
     if (c.np > 0)
@@ -3499,16 +3543,21 @@ void launch_sort_rest(Ctx &c, bool touched_list) {
     const int ncell = c.P.T * c.P.T * c.P.T;
     size_t sm = sizeof(int) * (3 * ncell + kSortCap);
     EXG_CUDA_OK(cudaFuncSetAttribute(k_tile_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    static int sgrid = 0;
-    if (!sgrid) sgrid = persistent_grid(k_tile_sort, sm);
+    // A tile's sort is a chain of passes over its particles, so while there are
+    // fewer tiles than blocks at a time a tile gets a block of 1024 threads (15
+    // thousand particles 28 -> 11 us, 1.1 M 34 -> 23 us); otherwise 256, of
+    // which more fit an SM.
+    const bool few = c.np < 148ll * 8 * 512 * 2;
+    const int thr = few ? 1024 : kThreads;
+    const int sgrid = persistent_grid(k_tile_sort, sm, thr);
     // no more blocks than the scene has tiles (small scenes of a batch)
     const int tgrid = (int)std::min<long long>(sgrid, c.P.ntiles);
-    k_tile_sort<<<tgrid, kThreads, sm, c.stream>>>(c.sb.active, c.sb.tile_start, c.sb.tile_count, c.sb.key,
+    k_tile_sort<<<tgrid, thr, sm, c.stream>>>(c.sb.active, c.sb.tile_start, c.sb.tile_count, c.sb.key,
                                                     c.sb.bucket, c.sb.bucket + c.cap, c.sb.perm, c.sb.cell_start, ncell,
                                                     c.ctl);
     if (touched_list)
-        k_touched<<<nblocks(c.P.ntiles), kThreads, 0, c.stream>>>(c.P, c.sb.tile_count, c.sb.touched,
-                                                                  c.sb.touched_step, c.ctl);
+        k_touched<<<nblocks(c.P.ntiles), kThreads, 0, c.stream>>>(c.P, c.sb.tile_count, c.sb.touched, c.sb.touched_step,
+                                                                  c.ctl, stencil_cells(c), scale_bits(c), bounds);
     EXG_CUDA_OK(cudaGetLastError());
 }
 
@@ -3518,18 +3567,12 @@ void launch_dt_finalize(Ctx &c, bool reset) {
 }
 
 void launch_scales_from(Ctx &c, const unsigned long long *bounds) {
-    const int W = (c.P.uniform_order == 1) ? 2 : (c.P.dual ? 3 : 4);
-    k_scales<<<1, 32, 0, c.stream>>>(c.ctl, W * W * W, c.precision == EXG_PREC_FP64 ? kFxBits64 : kFxBits32, bounds);
+    k_scales<<<1, 32, 0, c.stream>>>(c.ctl, stencil_cells(c), scale_bits(c), bounds);
     EXG_CUDA_OK(cudaGetLastError());
 }
 
 void launch_reset_accum(Ctx &c, unsigned long long *bounds, unsigned long long *dtmin) {
     k_reset_accum<<<1, 32, 0, c.stream>>>(bounds, dtmin);
-    EXG_CUDA_OK(cudaGetLastError());
-}
-
-void launch_time_advance(Ctx &c) {
-    k_time_advance<<<1, 1, 0, c.stream>>>(c.ctl);
     EXG_CUDA_OK(cudaGetLastError());
 }
 
@@ -3691,10 +3734,9 @@ void EXG_SFX(launch_g2p_fused)(Ctx &c, int mode) {
     }
 }
 
-void EXG_SFX(launch_copy_lost)(Ctx &c) {
-    if (c.np == 0) return;
-    k_copy_lost<EXG_R><<<nblocks(c.np), kThreads, 0, c.stream>>>(c.A<EXG_R>(), c.Bp<EXG_R>(), c.sb.key, c.np, c.ctl,
-                                                                 c.specs.use_temp);
+void EXG_SFX(launch_step_end)(Ctx &c) {
+    k_step_end<EXG_R><<<std::min(nblocks(std::max(c.np, 1ll)), 148 * 4), kThreads, 0, c.stream>>>(
+        c.A<EXG_R>(), c.Bp<EXG_R>(), c.sb.key, c.np, c.ctl, c.specs.use_temp);
     EXG_CUDA_OK(cudaGetLastError());
 }
 
