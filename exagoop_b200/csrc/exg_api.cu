@@ -623,6 +623,12 @@ void enqueue_step(Ctx &c) {
     if (c.timing) EXG_CUDA_OK(cudaEventRecord(c.ev[4], c.stream));
 }
 
+// The nodes near a body, after a level set was set (on the context's stream).
+void mark_near_bodies(Ctx &c) {
+    if (!c.ls_near) c.ls_near = dalloc<uint8_t>(c.P.nnodes);
+    launch_ls_near(c);
+}
+
 void swap_parts(Ctx &c) {
     std::swap(c.pa, c.pb);
     c.orient ^= 1;
@@ -784,6 +790,7 @@ int exg_ctx_destroy(exg_ctx *ctx) {
         delete reinterpret_cast<Nodes<float> *>(c.nodes);
     }
     for (double *p : c.ls) cudaFree(p);
+    cudaFree(c.ls_near);
     for (auto &row : c.udf_tab)
         for (double *p : row) cudaFree(p);
     for (auto &row : c.udfT_tab)
@@ -868,6 +875,7 @@ int exg_levelset_build_device(exg_ctx *ctx, int body, const exg_ls_shape *shapes
                                                        c.specs.plo[1], c.specs.plo[2], dx[0], dx[1], dx[2],
                                                        c.ls[body]);
         EXG_CUDA_OK(cudaGetLastError());
+        mark_near_bodies(c);
         EXG_CUDA_OK(cudaStreamSynchronize(c.stream));
         drop_graphs(c);
     });
@@ -914,7 +922,9 @@ int exg_set_levelset(exg_ctx *ctx, int body, const double *phi) {
     Ctx &c = ctx->c;
     EXG_TRY(ctx, {
         if (!c.ls[body]) c.ls[body] = dalloc<double>(c.P.nnodes);
-        EXG_CUDA_OK(cudaMemcpy(c.ls[body], phi, sizeof(double) * c.P.nnodes, cudaMemcpyHostToDevice));
+        EXG_CUDA_OK(cudaMemcpyAsync(c.ls[body], phi, sizeof(double) * c.P.nnodes, cudaMemcpyHostToDevice, c.stream));
+        mark_near_bodies(c);
+        EXG_CUDA_OK(cudaStreamSynchronize(c.stream));
         drop_graphs(c);
     });
     return EXG_OK;

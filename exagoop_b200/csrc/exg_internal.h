@@ -78,6 +78,7 @@ void d2h_int(Ctx &c, const void *src, int bytes, const int32_t *pid, int32_t *ho
 void upload_tables_fp64();
 void upload_tables_fp32();
 void launch_step_start(Ctx &c);
+void launch_ls_near(Ctx &c);
 void launch_keys(Ctx &c, bool zero_counts);
 // touched_list: also the list of tiles the nodal kernel writes and, from
 // bounds when given, the P2G's fixed-point scales
@@ -176,6 +177,7 @@ struct Ctx {
     void *nodes = nullptr;             // Nodes<R> host copy (device pointers)
     std::vector<void *> node_allocs;
     double *ls[kMaxBodies] = {};       // nodal level sets (FP64)
+    uint8_t *ls_near = nullptr;        // nodes near a body (NodeBCArgs::near)
     // UDF wall tables [lo/hi][dir] (FP64)
     double *udf_tab[2][3] = {};
     std::vector<double> udf_host[2][3];

@@ -1033,6 +1033,9 @@ struct NodeBCArgs {
     const double *udf[2][3];
     const double *ls[kMaxBodies];
     const double *udfT[2][3];  // wall-temperature tables: (value, second value) per face node
+    // per node: 0 where no level set within two nodes can be sampled below
+    // zero (ls_far), so that bodies are looked at only near them
+    const uint8_t *near;
 };
 
 __device__ __forceinline__ double ls_node_value(const Params &P, const double *phi, int i, int j, int k) {
@@ -1076,6 +1079,37 @@ __device__ void ls_sample(const Params &P, const double *phi, const double x[3],
         g[1] += ph * (w[0][o[0]] * dv[1][o[1]] * w[2][o[2]]);
         g[2] += ph * (w[0][o[0]] * w[1][o[1]] * dv[2][o[2]]);
     }
+}
+
+// Whether a node's level-set value alone cannot bring a sample below zero: a
+// sample is a combination of eight node values with weights in [0, 1] up to
+// rounding (1e-15), so values of 1e-6 dx .. 1e6 dx sum to well above zero.
+__device__ __forceinline__ bool ls_far(const Params &P, double phi) {
+    return phi >= 1e-6 * P.dxmin && phi <= 1e6 * P.dxmin;
+}
+// NodeBCArgs::near of every node: the 5 x 5 x 5 nodes around it, which hold
+// every corner a sample at the node or in the cell above it reads, whichever
+// way the position's cell index rounds.
+[[maybe_unused]] __global__ void k_ls_near(const __grid_constant__ Params P, const __grid_constant__ NodeBCArgs bc, uint8_t *near) {
+    const long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (n >= P.nnodes) return;
+    const int i = (int)(n % P.nn[0]), j = (int)((n / P.nn[0]) % P.nn[1]), k = (int)(n / ((long long)P.nn[0] * P.nn[1]));
+    bool far = true;
+    for (int b = 0; b < P.num_bodies && far; ++b) {
+        if (!bc.ls[b]) continue;
+        for (int q = 0; q < 125 && far; ++q)
+            far = ls_far(P, ls_node_value(P, bc.ls[b], i + q % 5 - 2, j + q / 5 % 5 - 2, k + q / 25 - 2));
+    }
+    near[n] = !far;
+}
+// Whether a particle at x has to look at the bodies.
+__device__ __forceinline__ bool ls_near(const Params &P, const NodeBCArgs &bc, const double x[3]) {
+    if (!bc.near) return false;  // no body has a level set
+    int c[3];
+    cell_of(P, x, c);
+    for (int d = 0; d < 3; ++d)
+        if (c[d] < 0 || c[d] > P.nc[d]) return true;
+    return bc.near[((long long)c[2] * P.nn[1] + c[1]) * P.nn[0] + c[0]] != 0;
 }
 
 // Domain walls of one node (nodal_bcs): relvel_in accumulates the wall
@@ -1128,7 +1162,7 @@ __device__ void node_bcs(const Params &P, const NodeBCArgs &bc, int i, int j, in
         }
     }
     // level-set bodies
-    if (P.num_bodies > 0 && m > 0.0) {
+    if (P.num_bodies > 0 && m > 0.0 && bc.near && bc.near[((long long)k * P.nn[1] + j) * P.nn[0] + i]) {
         const double xn[3] = {P.plo[0] + i * P.dx[0], P.plo[1] + j * P.dx[1], P.plo[2] + k * P.dx[2]};
         for (int b = 0; b < P.num_bodies; ++b) {
             if (!bc.ls[b]) continue;
@@ -1827,7 +1861,7 @@ __device__ __forceinline__ void move_particle(const Params &P, const NodeBCArgs 
     for (int d = 0; d < 3; ++d) x[d] += (double)vp[d] * dt;
     double rin[3] = {(double)v[0], (double)v[1], (double)v[2]};
     double rout[3] = {rin[0], rin[1], rin[2]};
-    if (!LEAN && P.num_bodies > 0 && phase == 0) {
+    if (!LEAN && P.num_bodies > 0 && phase == 0 && ls_near(P, bc, x)) {
         int hit = -1;
         double minphi = kTiny;
         for (int b = 0; b < P.num_bodies; ++b) {
@@ -3506,10 +3540,16 @@ static NodeBCArgs make_bc(Ctx &c) {
             bc.udfT[s][d] = c.udfT_tab[s][d];
         }
     for (int b = 0; b < kMaxBodies; ++b) bc.ls[b] = c.ls[b];
+    bc.near = c.ls_near;
     return bc;
 }
 
 #if defined(EXG_R_FP64)
+void launch_ls_near(Ctx &c) {
+    k_ls_near<<<nblocks(c.P.nnodes), kThreads, 0, c.stream>>>(c.P, make_bc(c), c.ls_near);
+    EXG_CUDA_OK(cudaGetLastError());
+}
+
 static int stencil_cells(const Ctx &c) {
     const int W = (c.P.uniform_order == 1) ? 2 : (c.P.dual ? 3 : 4);
     return W * W * W;
