@@ -634,24 +634,28 @@ void swap_parts(Ctx &c) {
     c.orient ^= 1;
 }
 
-// Interleaved node records and the tensor map the fused G2P stages its node
-// blocks with (one 4-D box: record words x B x B x B).  Skipped on grids
-// with a periodic axis (the box cannot wrap) or when EXG_NO_TMA is set; the
-// G2P then stages with plain loads.
+// Interleaved node records, from which the fused G2P stages its node blocks, and
+// the tensor map to do so with one 4-D box (record words x B x B x B).  No
+// tensor map on grids with a periodic axis (the box cannot wrap) or when
+// EXG_NO_TMA is set: the G2P then stages with plain loads.
 void setup_node_records(Ctx &c) {
     std::memset(&c.tmap, 0, sizeof(c.tmap));
     c.tma = false;
-    if (c.P.periodic[0] || c.P.periodic[1] || c.P.periodic[2] || std::getenv("EXG_NO_TMA")) return;
     const bool f64 = fp64(c);
     const size_t esz = f64 ? 8 : 4, ns = f64 ? rec_words<double>() : rec_words<float>();
+    EXG_CUDA_OK(cudaMalloc(&c.rec, esz * ns * c.P.nnodes));
+    EXG_CUDA_OK(cudaMemset(c.rec, 0, esz * ns * c.P.nnodes));
+    if (f64)
+        reinterpret_cast<Nodes<double> *>(c.nodes)->rec = reinterpret_cast<double *>(c.rec);
+    else
+        reinterpret_cast<Nodes<float> *>(c.nodes)->rec = reinterpret_cast<float *>(c.rec);
+    if (c.P.periodic[0] || c.P.periodic[1] || c.P.periodic[2] || std::getenv("EXG_NO_TMA")) return;
     void *fn = nullptr;
     cudaDriverEntryPointQueryResult q;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || !fn ||
         q != cudaDriverEntryPointSuccess)
         return;
     auto encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-    EXG_CUDA_OK(cudaMalloc(&c.rec, esz * ns * c.P.nnodes));
-    EXG_CUDA_OK(cudaMemset(c.rec, 0, esz * ns * c.P.nnodes));
     const cuuint64_t dims[4] = {ns, (cuuint64_t)c.P.nn[0], (cuuint64_t)c.P.nn[1], (cuuint64_t)c.P.nn[2]};
     const cuuint64_t strides[3] = {esz * ns, esz * ns * c.P.nn[0], esz * ns * c.P.nn[0] * c.P.nn[1]};
     const cuuint32_t box[4] = {(cuuint32_t)ns, (cuuint32_t)c.P.B, (cuuint32_t)c.P.B, (cuuint32_t)c.P.B};
@@ -660,16 +664,7 @@ void setup_node_records(Ctx &c) {
                               c.rec, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        cudaFree(c.rec);
-        c.rec = nullptr;
-        return;
-    }
-    c.tma = true;
-    if (f64)
-        reinterpret_cast<Nodes<double> *>(c.nodes)->rec = reinterpret_cast<double *>(c.rec);
-    else
-        reinterpret_cast<Nodes<float> *>(c.nodes)->rec = reinterpret_cast<float *>(c.rec);
+    c.tma = r == CUDA_SUCCESS;
 }
 
 void drop_graphs(Ctx &c) {

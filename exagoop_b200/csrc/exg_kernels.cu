@@ -2013,7 +2013,7 @@ __device__ __forceinline__ void volume_stress(const Params &P, const Material &m
 template <class R>
 __device__ __forceinline__ bool all_finite(const R *a, int n) {
     bool ok = true;
-    for (int i = 0; i < n; ++i) ok = ok && isfinite((double)a[i]);
+    for (int i = 0; i < n; ++i) ok = ok && isfinite(a[i]);
     return ok;
 }
 
@@ -2073,15 +2073,18 @@ __device__ __forceinline__ void g2p_tile(const SplineTables *tab, R *nb, const P
     na.B3 = B3;
     for (int d = 0; d < 3; ++d) na.org[d] = tc[d] * P.T - P.hlo;
     if (!staged) {
-        // the node block by plain loads (the caller did not stage it by TMA)
+        // the node block by plain loads (the caller did not stage it by TMA),
+        // from the nodal kernel's records: a node is two (FP64 three) 16-byte
+        // loads instead of one from each of six arrays
+        constexpr int NS = SmemNodes<R>::NS;
         for (int idx = threadIdx.x; idx < B3; idx += blockDim.x) {
             const int bx = idx % B, by = (idx / B) % B, bz = idx / (B * B);
             const long long ni = node_index(P, na.org[0] + bx, na.org[1] + by, na.org[2] + bz);
-            R *q = nb + idx * SmemNodes<R>::NS;
-            for (int c = 0; c < 3; ++c) {
-                q[c] = ni >= 0 ? Nd.c[EXG_N_VEL + c][ni] : R(0);
-                q[3 + c] = ni >= 0 ? Nd.c[EXG_N_DVEL + c][ni] : R(0);
-            }
+            const float4 *src = reinterpret_cast<const float4 *>(Nd.rec + max(ni, 0ll) * NS);
+            float4 *dst = reinterpret_cast<float4 *>(nb + idx * NS);
+#pragma unroll
+            for (int q = 0; q < NS * (int)sizeof(R) / 16; ++q)
+                dst[q] = ni >= 0 ? src[q] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         __syncthreads();
     }
