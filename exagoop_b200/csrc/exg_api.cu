@@ -358,7 +358,9 @@ void p2g_split(Ctx &c, long long n, long long np) {
     }
     int gs = kG2PMaxShift;
     while (gs > kG2PMinShift && (n >> gs) < (c.tma ? kG2PItems : kG2PItemsPlain)) --gs;
-    if (ps != c.P.pshift || gs != c.P.gshift) drop_graphs(c);
+    const int small = n < kSmallScene;
+    if (ps != c.P.pshift || gs != c.P.gshift || small != c.P.small) drop_graphs(c);
+    c.P.small = small;
     c.P.gshift = gs;
     c.P.pshift = ps;
     c.P.Bz = (c.P.T >> ps) + c.P.hlo + c.P.hhi;

@@ -57,7 +57,7 @@ struct Ctl {
     int n_touched_tiles;
     long long n_sorted;                // particles inside the domain after the sort
     unsigned long long lost_fill;      // next slot for out-of-domain particles in the re-ordered storage
-    int next_p2g;                      // dynamic tile counter of the P2G kernel (reset by k_scales)
+    int next_p2g;                      // dynamic tile counter of the P2G kernel (reset with the fixed-point scales)
     int next_g2p;                      // dynamic item counter of the fused G2P (reset by k_nodes)
     int n_g2p_items;                   // work items of the fused G2P
     int pad2;
@@ -70,6 +70,7 @@ struct Ctl {
 // 8^3 tile) stay whole: items of 1024 made the 9 M-particle sphere step's G2P
 // 5 % slower (FP64, whose node block arrives single-buffered, 15 %).
 constexpr int kG2PMaxShift = 12, kG2PMinShift = 8;
+constexpr long long kSmallScene = 1 << 16;
 
 // Per-tile stride of the P2G staging array, in 64-bit words, for nv
 // fixed-point values: FP32 state one 64-bit integer per value; FP64 state
@@ -127,6 +128,7 @@ struct Params {
     // the W x W columns a warp adds to over more shared-memory banks
     int PS;
     int gshift;         // log2 of the particles of a fused-G2P work item
+    int small;          // fewer than kSmallScene particles in a launch (step_early)
     double gravity[3];
     int external_loads;
     double slab_lo[3], slab_hi[3], extforce[3];

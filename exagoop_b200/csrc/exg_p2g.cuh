@@ -438,6 +438,7 @@ __device__ __forceinline__ void p2g_run(const Src &src, unsigned char *smraw, P2
     load_tables(tab);
     for (int i = threadIdx.x; i < (int)(2 * p2g_buf_bytes<R>(nv) / 16); i += blockDim.x)
         reinterpret_cast<uint4 *>(accs)[i] = make_uint4(0u, 0u, 0u, 0u);
+    step_kernel_begin(src.early());
     const int lane = threadIdx.x & 31;
     const Ln ln;
     const int sy = ln.yz % W, sz = ln.yz / W;
@@ -642,11 +643,12 @@ struct P2GScene {
     const int32_t *pm;
     long long *stg;
     Ctl *c;
-    int nitems;
+    int pshift;
     __device__ __forceinline__ int take(int &) const {
         const int i = atomicAdd(&c->next_p2g, 1);
-        return i < nitems ? i : -1;
+        return i < c->n_active_tiles << pshift ? i : -1;
     }
+    __device__ __forceinline__ bool early() const { return step_early(P); }
     __device__ __forceinline__ const Params &params(int) const { return P; }
     __device__ __forceinline__ const Parts<R> &parts(int) const { return A; }
     __device__ __forceinline__ const int *active(int) const { return act; }
@@ -664,6 +666,6 @@ __global__ void __launch_bounds__(P2GVar<R, ORD, V>::THREADS, 1)
           const int *cell_start, const int32_t *perm, long long *staging, Ctl *ctl) {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ P2GBuf bufs[2];
-    const P2GScene<R> src{P, A, active, start, cell_start, perm, staging, ctl, ctl->n_active_tiles << P.pshift};
+    const P2GScene<R> src{P, A, active, start, cell_start, perm, staging, ctl, P.pshift};
     p2g_run<R, ORD, THERM>(src, smraw, bufs, p2g_values<THERM>(P), P.pshift);
 }
