@@ -366,8 +366,8 @@ int exg_get_stream(exg_ctx *ctx, void **stream);
  * No counterpart in the reference, whose only tiling knob is
  * mpm.max_grid_size (the box size of its BoxArray, Source/mpm_init.cpp:
  * 154-155).  The P2G and the fused G2P kernels each come in EXG_NUM_VARIANTS
- * launch variants (P2G: rows of the stencil slice per pass and threads per
- * block; G2P: threads per block and resident blocks per SM).  Every variant
+ * launch variants (P2G: threads per block; G2P: threads per block and
+ * resident blocks per SM).  Every variant
  * gives bit-identical results; only their speed differs with the GPU, the
  * B-spline order, the precision and the particle distribution.
  * exg_autotune times each variant on the context's current particles (a few
