@@ -327,18 +327,28 @@ void upload_parts(Ctx &c, const exg_particle_soa *h, const std::vector<int32_t> 
 
 void drop_graphs(Ctx &c);
 
-// Work split of the P2G and the fused G2P for launches over n particles (of all
-// scenes of a batch), np of them this scene's: a tile's P2G is cut into
-// 1 << pshift items, the fused G2P works on 1 << gshift particles at a time.
-// Makes the P2G's staging array hold its items.
-void p2g_split(Ctx &c, long long n, long long np) {
-    const bool f64 = fp64(c);
-    // staging words for a split: no more tiles hold particles than there are
-    // particles
+// 64-bit words of the staging array for the context's tiles split by ps: no
+// more tiles hold particles than there are particles.
+size_t staging_words(const Ctx &c, int ps) {
+    const long long nv = ((long long)c.nch * c.P.PS * ((c.P.T >> ps) + c.P.hlo + c.P.hhi) + 3) & ~3ll;
+    const long long tiles = std::min(c.P.ntiles, std::max(1ll, c.np)) << ps;
+    return (size_t)(tiles * (fp64(c) ? stg_stride<double>(nv) : stg_stride<float>(nv)));
+}
+
+// Work split of the P2G and the fused G2P for launches that cover all of the
+// given scenes (one, or those of a batch, which share the order, the tile and
+// the precision): a tile's P2G is cut into 1 << pshift items, the fused G2P
+// works on 1 << gshift particles at a time.  One pshift for all scenes: the
+// batched P2G has one node-block layout for the launch.  Makes each scene's
+// staging array hold its items.
+void p2g_split(const std::vector<Ctx *> &scenes) {
+    const Ctx &c = *scenes[0];
+    long long n = 0;
+    for (const Ctx *x : scenes) n += x->np;
     auto words = [&](int ps) {
-        const long long nv = ((long long)c.nch * c.P.PS * ((c.P.T >> ps) + c.P.hlo + c.P.hhi) + 3) & ~3ll;
-        const long long tiles = std::min(c.P.ntiles, std::max(1ll, np)) << ps;
-        return (size_t)(tiles * (f64 ? stg_stride<double>(nv) : stg_stride<float>(nv)));
+        size_t w = 0;
+        for (const Ctx *x : scenes) w += staging_words(*x, ps);
+        return w;
     };
     int ps = 0;
     const long long tiles = std::max<long long>(1, n / (8ll * c.P.T * c.P.T * c.P.T));
@@ -348,22 +358,24 @@ void p2g_split(Ctx &c, long long n, long long np) {
     while (ps > 0 && words(ps) > std::max(2 * words(0), (size_t)8 << 20)) --ps;
     // a block holds two node blocks and the records of its warps
     while (ps < c.P.tshift && !DISPATCH(p2g_fits, c, ps)) ++ps;
-    if (words(ps) > c.staging_cap) {
-        cudaFree(c.staging);
-        c.staging = nullptr;
-        c.staging_cap = 0;
-        c.staging = dalloc<long long>(words(ps));
-        c.staging_cap = words(ps);
-        drop_graphs(c);
-    }
-    int gs = kG2PMaxShift;
-    while (gs > kG2PMinShift && (n >> gs) < (c.tma ? kG2PItems : kG2PItemsPlain)) --gs;
     const int small = n < kSmallScene;
-    if (ps != c.P.pshift || gs != c.P.gshift || small != c.P.small) drop_graphs(c);
-    c.P.small = small;
-    c.P.gshift = gs;
-    c.P.pshift = ps;
-    c.P.Bz = (c.P.T >> ps) + c.P.hlo + c.P.hhi;
+    for (Ctx *x : scenes) {
+        if (staging_words(*x, ps) > x->staging_cap) {
+            cudaFree(x->staging);
+            x->staging = nullptr;
+            x->staging_cap = 0;
+            x->staging = dalloc<long long>(staging_words(*x, ps));
+            x->staging_cap = staging_words(*x, ps);
+            drop_graphs(*x);
+        }
+        int gs = kG2PMaxShift;
+        while (gs > kG2PMinShift && (n >> gs) < (x->tma ? kG2PItems : kG2PItemsPlain)) --gs;
+        if (ps != x->P.pshift || gs != x->P.gshift || small != x->P.small) drop_graphs(*x);
+        x->P.small = small;
+        x->P.gshift = gs;
+        x->P.pshift = ps;
+        x->P.Bz = (x->P.T >> ps) + x->P.hlo + x->P.hhi;
+    }
 }
 
 }  // namespace
@@ -1017,10 +1029,10 @@ int exg_particles_upload(exg_ctx *ctx, const exg_particle_soa *p) {
         }
         EXG_CUDA_OK(cudaMemcpy(c.mat_dev, c.mats.data(), sizeof(Material) * c.mats.size(), cudaMemcpyHostToDevice));
         const bool temp = c.specs.use_temp != 0;
-        p2g_split(c, n, n);
         if (g2p_lean(c) != lean_before) drop_graphs(c);  // the graphs hold the other G2P variant
         if (c.pa && n == c.np && n == c.cap) {
             // same particle count: the storage, sort buffers and step graphs stay
+            p2g_split({&c});
             if (fp64(c))
                 upload_parts<double>(c, p, mat);
             else
@@ -1072,6 +1084,7 @@ int exg_particles_upload(exg_ctx *ctx, const exg_particle_soa *p) {
         c.sb.key = dalloc<uint32_t>(n);
         c.sb.perm = dalloc<int32_t>(n);
         c.sb.bucket = dalloc<int32_t>(2 * n);
+        p2g_split({&c});
         c.parts_sorted = false;
         c.reordered = false;
         c.reduce_stale = true;
@@ -1904,9 +1917,7 @@ int exg_batch_step(exg_batch *B, int nsteps) {
     try {
         for (Ctx *c : b.scenes)
             if (c->reduce_stale) do_reduce(*c);
-        long long total = 0;
-        for (Ctx *c : b.scenes) total += c->np;
-        for (Ctx *c : b.scenes) p2g_split(*c, total, c->np);  // one split for all: the launch covers every scene
+        p2g_split(b.scenes);
         const bool changed = b.precision == EXG_PREC_FP64 ? batch_descriptors_fp64(b) : batch_descriptors_fp32(b);
         int lean = 1;
         for (Ctx *sc : b.scenes) lean = lean && g2p_lean(*sc);

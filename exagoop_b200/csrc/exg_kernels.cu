@@ -3972,6 +3972,12 @@ void d2h_int(Ctx &c, const void *src, int bytes, const int32_t *pid, int32_t *ho
 template <class R>
 static bool batch_descriptors_t(Batch &b) {
     const size_t n = b.scenes.size();
+    // the batched P2G takes the split and the node-block layout of the launch
+    // from the first scene, the nodal kernel each scene's own
+    const Params &P0 = b.scenes[0]->P;
+    for (const Ctx *c : b.scenes)
+        if (c->P.pshift != P0.pshift || c->P.Bz != P0.Bz || c->P.PS != P0.PS || c->P.T != P0.T)
+            throw std::runtime_error("internal: the scenes of a batch have different P2G work splits");
     bool changed = false;
     for (int par = 0; par < 2; ++par) {
         std::vector<SceneDesc<R>> d(n);

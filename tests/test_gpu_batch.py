@@ -63,6 +63,28 @@ def test_batch_matches_single_contexts(precision):
     b.close()
 
 
+@pytest.mark.parametrize("precision", [nt.PREC_FP64, nt.PREC_MIXED])
+@pytest.mark.parametrize("order", [2, 3])
+@pytest.mark.parametrize("sides", [(32, 56), (56, 32)])
+def test_batch_scenes_of_unequal_staging(sides, order, precision):
+    """A small and a larger grid with few particles: alone the small one's
+    tiles would be split finer than the larger one's (whose staging array is
+    the limit), the batch needs one split for both."""
+    items = []
+    for n in sides:
+        s, p = scenes.dam_break(n=(n, n, n), size=(1.0, 1.0, 1.0), block=(0.4, 0.5, 0.4), seed=n, precision=precision,
+                                order=order)
+        items.append((s, p, None))
+    assert sum(p.n for _, p, _ in items) < 444 * 8 * 8 ** 3 // 4
+    b, got = run_batch(items, 6)
+    for i, (s, p, phi) in enumerate(items):
+        ctx, ref = run_single(s, p, phi, 6)
+        assert np.array_equal(got[i].rdata, ref.rdata), f"scene {i}"
+        assert np.array_equal(got[i].pos, ref.pos), f"scene {i}"
+        ctx.close()
+    b.close()
+
+
 def test_batch_matches_oracle():
     items = uneven_scenes(nt.PREC_FP64)
     b, got = run_batch(items, 10)
