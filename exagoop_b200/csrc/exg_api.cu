@@ -335,12 +335,21 @@ size_t staging_words(const Ctx &c, int ps) {
     return (size_t)(tiles * (fp64(c) ? stg_stride<double>(nv) : stg_stride<float>(nv)));
 }
 
+// Frees the staging array, with the step graphs that hold its address.
+void drop_staging(Ctx &c) {
+    drop_graphs(c);
+    cudaFree(c.staging);
+    c.staging = nullptr;
+    c.staging_cap = 0;
+}
+
 // Work split of the P2G and the fused G2P for launches that cover all of the
 // given scenes (one, or those of a batch, which share the order, the tile and
 // the precision): a tile's P2G is cut into 1 << pshift items, the fused G2P
 // works on 1 << gshift particles at a time.  One pshift for all scenes: the
 // batched P2G has one node-block layout for the launch.  Makes each scene's
-// staging array hold its items.
+// staging array hold its items.  Where the memory for that is not to be had it
+// throws and the scene is left without one (need_staging).
 void p2g_split(const std::vector<Ctx *> &scenes) {
     const Ctx &c = *scenes[0];
     long long n = 0;
@@ -360,13 +369,19 @@ void p2g_split(const std::vector<Ctx *> &scenes) {
     while (ps < c.P.tshift && !DISPATCH(p2g_fits, c, ps)) ++ps;
     const int small = n < kSmallScene;
     for (Ctx *x : scenes) {
-        if (staging_words(*x, ps) > x->staging_cap) {
-            cudaFree(x->staging);
-            x->staging = nullptr;
-            x->staging_cap = 0;
-            x->staging = dalloc<long long>(staging_words(*x, ps));
-            x->staging_cap = staging_words(*x, ps);
-            drop_graphs(*x);
+        const size_t need = staging_words(*x, ps);
+        if (need > x->staging_cap) {
+            drop_staging(*x);
+            try {
+                if (need > x->staging_max)
+                    throw std::runtime_error("the P2G staging array needs " + std::to_string(8 * need) +
+                                             " bytes, EXG_P2G_STAGING_MAX is " + std::to_string(8 * x->staging_max));
+                x->staging = dalloc<long long>(need);
+            } catch (...) {
+                cudaGetLastError();  // or the next launch would report it
+                throw;
+            }
+            x->staging_cap = need;
         }
         int gs = kG2PMaxShift;
         while (gs > kG2PMinShift && (n >> gs) < (x->tma ? kG2PItems : kG2PItemsPlain)) --gs;
@@ -376,6 +391,12 @@ void p2g_split(const std::vector<Ctx *> &scenes) {
         x->P.pshift = ps;
         x->P.Bz = (x->P.T >> ps) + x->P.hlo + x->P.hhi;
     }
+}
+
+// Before a P2G: a context whose last upload (or batch step) found no memory for
+// the staging array has none, and tries again here.
+void need_staging(Ctx &c) {
+    if (!c.staging) p2g_split({&c});
 }
 
 }  // namespace
@@ -708,6 +729,7 @@ int exg_ctx_create(const exg_specs *specs, int device, exg_ctx **out) {
         c.specs = *specs;
         c.precision = specs->precision;
         c.timing = std::getenv("EXG_STAGE_TIMING") != nullptr;
+        if (const char *most = std::getenv("EXG_P2G_STAGING_MAX")) c.staging_max = std::strtoull(most, nullptr, 10) / 8;
         c.device = device;
         EXG_CUDA_OK(cudaSetDevice(device));
         EXG_CUDA_OK(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
@@ -1032,7 +1054,6 @@ int exg_particles_upload(exg_ctx *ctx, const exg_particle_soa *p) {
         if (g2p_lean(c) != lean_before) drop_graphs(c);  // the graphs hold the other G2P variant
         if (c.pa && n == c.np && n == c.cap) {
             // same particle count: the storage, sort buffers and step graphs stay
-            p2g_split({&c});
             if (fp64(c))
                 upload_parts<double>(c, p, mat);
             else
@@ -1042,6 +1063,7 @@ int exg_particles_upload(exg_ctx *ctx, const exg_particle_soa *p) {
             c.reordered = false;
             c.reduce_stale = true;
             sync(c);
+            p2g_split({&c});
             return EXG_OK;
         }
         // particle storage (re-allocated when the count changes)
@@ -1084,11 +1106,11 @@ int exg_particles_upload(exg_ctx *ctx, const exg_particle_soa *p) {
         c.sb.key = dalloc<uint32_t>(n);
         c.sb.perm = dalloc<int32_t>(n);
         c.sb.bucket = dalloc<int32_t>(2 * n);
-        p2g_split({&c});
         c.parts_sorted = false;
         c.reordered = false;
         c.reduce_stale = true;
         sync(c);
+        p2g_split({&c});
     });
     return EXG_OK;
 }
@@ -1228,6 +1250,7 @@ int exg_p2g_momentum(exg_ctx *ctx, int update_mass, int update_vel, int update_f
     Ctx &c = ctx->c;
     if (c.np == 0) return fail(ctx, EXG_ERR_NOT_READY, "no particles");
     EXG_TRY(ctx, {
+        need_staging(c);
         int flags = (update_mass ? PF_MASS : 0) | (update_vel ? PF_VEL : 0) | (update_forces ? PF_FORCE : 0);
         EXG_CUDA_OK(cudaMemsetAsync(&c.ctl->maxppc, 0, sizeof(int), c.stream));
         do_sort(c, false);
@@ -1358,6 +1381,7 @@ int exg_p2g_temperature(exg_ctx *ctx, int reset, int update_temp, int update_sou
     if (!reset)
         return fail(ctx, EXG_ERR_UNSUPPORTED, "P2G_Temperature without reset (the reference always resets)");
     EXG_TRY(ctx, {
+        need_staging(c);
         const int flags = (update_temp ? PF_TEMP : 0) | (update_source ? PF_SRC : 0);
         EXG_CUDA_OK(cudaMemsetAsync(&c.ctl->maxppc, 0, sizeof(int), c.stream));
         do_sort(c, false);
@@ -1540,6 +1564,7 @@ int exg_autotune(exg_ctx *ctx) {
     Ctx &c = ctx->c;
     if (c.np == 0) return fail(ctx, EXG_ERR_NOT_READY, "no particles");
     EXG_TRY(ctx, {
+        need_staging(c);
         const int p0 = c.p2g_var, g0 = c.g2p_var;
         autotune_impl(c);
         if (c.p2g_var != p0 || c.g2p_var != g0) drop_graphs(c);
@@ -1576,6 +1601,7 @@ int exg_step(exg_ctx *ctx, int nsteps) {
     Ctx &c = ctx->c;
     if (c.np == 0) return fail(ctx, EXG_ERR_NOT_READY, "no particles");
     EXG_TRY(ctx, {
+        need_staging(c);
         const bool tune = c.specs.autotune && nsteps > 0;
         if (tune) ensure_tuned(c);
         if (c.reduce_stale) do_reduce(c);

@@ -193,6 +193,7 @@ struct Ctx {
     double *stage = nullptr;           // one FP64 particle field: host transfers
     long long stage_cap = 0;
     size_t staging_cap = 0;            // in 64-bit words
+    size_t staging_max = ~(size_t)0;   // most words it may take (EXG_P2G_STAGING_MAX, in bytes, at creation)
     int nch = 7;
     // control block
     Ctl *ctl = nullptr;                // device

@@ -259,3 +259,33 @@ def test_lattice_start_paths(case, precision):
         T = r.rdata[nt.R_TEMPERATURE]
         eT = np.linalg.norm(g.rdata[nt.R_TEMPERATURE] - T) / np.linalg.norm(T)
         assert eT < (1e-12 if precision == "fp64" else 1e-5), eT
+
+
+def test_no_memory_for_the_staging_array(monkeypatch):
+    # the P2G's staging array grows with the upload; where its memory is not
+    # to be had (here: a limit between what 2 and 6000 particles need), the
+    # calls that would use it report that, and a later upload recovers
+    s, dx = unit_box(3)
+    rng = np.random.default_rng(3)
+    few, many = (elastic(rng.uniform(0.1, 0.9, (3, n)), dx, 3) for n in (2, 6000))
+    monkeypatch.setenv("EXG_P2G_STAGING_MAX", str(1 << 20))
+    ctx = nt.Context(s)
+    ctx.upload(few)
+    ctx.Initialise_Internal_Forces()
+    ctx.step(4)  # two of them replayed from graphs
+    with pytest.raises(nt.ExgError, match="staging"):
+        ctx.upload(many)
+    for call in (lambda: ctx.step(1), lambda: ctx.P2G_Momentum(1, 1, 1), lambda: ctx.autotune()):
+        with pytest.raises(nt.ExgError, match="staging"):
+            call()
+    ctx.upload(few)
+    ctx.Initialise_Internal_Forces()
+    ctx.step(4)
+    fresh = nt.Context(s)
+    fresh.upload(few)
+    fresh.Initialise_Internal_Forces()
+    fresh.step(4)
+    a, b = ctx.download(), fresh.download()
+    assert np.array_equal(a.pos, b.pos) and np.array_equal(a.rdata, b.rdata)
+    ctx.close()
+    fresh.close()
