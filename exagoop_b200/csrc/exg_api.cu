@@ -175,7 +175,8 @@ void build_params_for(const exg_specs &s, Params &P) {
     P.pshift = 0;
     P.gshift = kG2PMaxShift;
     P.Bz = P.B;
-    P.PS = P.B == 11 ? 130 : P.B * P.B;  // 130: 2 mod 32, the 4 x 4 columns of a cubic row on 16 banks
+    P.PS = P.B * P.B;
+    P.nbuf = 1;
     for (int d = 0; d < 3; ++d)
         P.ntile[d] = s.periodic[d] ? s.ncells[d] / T : (s.ncells[d] + 1 + T - 1) / T;
     P.ntiles = (long long)P.ntile[0] * P.ntile[1] * P.ntile[2];
@@ -327,11 +328,11 @@ void upload_parts(Ctx &c, const exg_particle_soa *h, const std::vector<int32_t> 
 
 void drop_graphs(Ctx &c);
 
-// 64-bit words of the staging array for the context's tiles split by ps: no
-// more tiles hold particles than there are particles.
-size_t staging_words(const Ctx &c, int ps) {
-    const long long nv = ((long long)c.nch * c.P.PS * ((c.P.T >> ps) + c.P.hlo + c.P.hhi) + 3) & ~3ll;
-    const long long tiles = std::min(c.P.ntiles, std::max(1ll, c.np)) << ps;
+// 64-bit words of the staging array for the context's tiles: no more tiles
+// hold particles than there are particles.
+size_t staging_words(const Ctx &c, const P2GSplit &s) {
+    const long long nv = ((long long)c.nch * s.PS * ((c.P.T >> s.pshift) + c.P.hlo + c.P.hhi) + 3) & ~3ll;
+    const long long tiles = std::min(c.P.ntiles, std::max(1ll, c.np)) << s.pshift;
     return (size_t)(tiles * (fp64(c) ? stg_stride<double>(nv) : stg_stride<float>(nv)));
 }
 
@@ -343,53 +344,83 @@ void drop_staging(Ctx &c) {
     c.staging_cap = 0;
 }
 
+// Makes the staging array hold the context's items.
+void fit_staging(Ctx &c, const P2GSplit &s) {
+    const size_t need = staging_words(c, s);
+    if (need <= c.staging_cap) return;
+    drop_staging(c);
+    if (need > c.staging_max)
+        throw std::runtime_error("the P2G staging array needs " + std::to_string(8 * need) +
+                                 " bytes, EXG_P2G_STAGING_MAX is " + std::to_string(8 * c.staging_max));
+    c.staging = dalloc<long long>(need);
+    c.staging_cap = need;
+}
+
 // Work split of the P2G and the fused G2P for launches that cover all of the
 // given scenes (one, or those of a batch, which share the order, the tile and
 // the precision): a tile's P2G is cut into 1 << pshift items, the fused G2P
-// works on 1 << gshift particles at a time.  One pshift for all scenes: the
+// works on 1 << gshift particles at a time.  One split for all scenes: the
 // batched P2G has one node-block layout for the launch.  Makes each scene's
 // staging array hold its items.  Where the memory for that is not to be had it
-// throws and the scene is left without one (need_staging).
+// throws and the scenes are left without one (need_staging).
 void p2g_split(const std::vector<Ctx *> &scenes) {
     const Ctx &c = *scenes[0];
     long long n = 0;
     for (const Ctx *x : scenes) n += x->np;
-    auto words = [&](int ps) {
+    auto words = [&](const P2GSplit &s) {
         size_t w = 0;
-        for (const Ctx *x : scenes) w += staging_words(*x, ps);
+        for (const Ctx *x : scenes) w += staging_words(*x, s);
         return w;
     };
-    int ps = 0;
+    const int B2 = c.P.B * c.P.B;
+    // the least staging: whole tiles, one node block, no padding.  Where memory
+    // allows more it is mostly slower: P2G and nodal kernel together 634 -> 709
+    // us for 2.2 M FP64 cubic particles, 310 -> 334 in FP32, 1544 -> 1726 for
+    // 2.8 M FP64 with temperature (FP32 530 -> 502), 102 -> 165 for 140 thousand
+    const P2GSplit least{0, 1, B2};
+    P2GSplit s{0, 2, c.P.B == 11 ? 130 : B2};  // 130: 2 mod 32, the 4 x 4 columns of a cubic row on 16 banks
+    const size_t whole = words(s);
     const long long tiles = std::max<long long>(1, n / (8ll * c.P.T * c.P.T * c.P.T));
-    while (ps < c.P.tshift && (tiles << ps) < kP2GItems) ++ps;
+    while (s.pshift < c.P.tshift && (tiles << s.pshift) < kP2GItems) ++s.pshift;
     // finer splits overlap more: at most twice the staging of whole tiles where
     // that is more than 64 MB
-    while (ps > 0 && words(ps) > std::max(2 * words(0), (size_t)8 << 20)) --ps;
+    while (s.pshift > 0 && words(s) > std::max(2 * whole, (size_t)8 << 20)) --s.pshift;
     // a block holds two node blocks and the records of its warps
-    while (ps < c.P.tshift && !DISPATCH(p2g_fits, c, ps)) ++ps;
+    while (s.pshift < c.P.tshift && !DISPATCH(p2g_fits, c, s)) ++s.pshift;
+    // which takes FP64 cubic with temperature to eighths, three times the
+    // staging of whole tiles: up to an eighth of the device's memory
+    if (words(s) > std::max(2 * whole, (size_t)8 << 20)) {
+        size_t mem_free = 0, mem = 0;
+        EXG_CUDA_OK(cudaMemGetInfo(&mem_free, &mem));
+        if (words(s) > mem / (8 * sizeof(long long))) s = least;
+    }
+    for (const Ctx *x : scenes)
+        if (x->least_staging) s = least;
+    for (;;) {
+        try {
+            for (Ctx *x : scenes) fit_staging(*x, s);
+            break;
+        } catch (...) {
+            cudaGetLastError();  // or the next launch would report it
+            for (Ctx *x : scenes) drop_staging(*x);
+            if (words(least) >= words(s)) throw;
+            s = least;
+            for (Ctx *x : scenes) x->least_staging = true;
+        }
+    }
     const int small = n < kSmallScene;
     for (Ctx *x : scenes) {
-        const size_t need = staging_words(*x, ps);
-        if (need > x->staging_cap) {
-            drop_staging(*x);
-            try {
-                if (need > x->staging_max)
-                    throw std::runtime_error("the P2G staging array needs " + std::to_string(8 * need) +
-                                             " bytes, EXG_P2G_STAGING_MAX is " + std::to_string(8 * x->staging_max));
-                x->staging = dalloc<long long>(need);
-            } catch (...) {
-                cudaGetLastError();  // or the next launch would report it
-                throw;
-            }
-            x->staging_cap = need;
-        }
+        Params &P = x->P;
         int gs = kG2PMaxShift;
         while (gs > kG2PMinShift && (n >> gs) < (x->tma ? kG2PItems : kG2PItemsPlain)) --gs;
-        if (ps != x->P.pshift || gs != x->P.gshift || small != x->P.small) drop_graphs(*x);
-        x->P.small = small;
-        x->P.gshift = gs;
-        x->P.pshift = ps;
-        x->P.Bz = (x->P.T >> ps) + x->P.hlo + x->P.hhi;
+        if (s.pshift != P.pshift || s.nbuf != P.nbuf || s.PS != P.PS || gs != P.gshift || small != P.small)
+            drop_graphs(*x);
+        P.small = small;
+        P.gshift = gs;
+        P.pshift = s.pshift;
+        P.nbuf = s.nbuf;
+        P.PS = s.PS;
+        P.Bz = (P.T >> s.pshift) + P.hlo + P.hhi;
     }
 }
 
@@ -1063,6 +1094,7 @@ int exg_particles_upload(exg_ctx *ctx, const exg_particle_soa *p) {
             c.reordered = false;
             c.reduce_stale = true;
             sync(c);
+            c.least_staging = false;
             p2g_split({&c});
             return EXG_OK;
         }
@@ -1110,6 +1142,7 @@ int exg_particles_upload(exg_ctx *ctx, const exg_particle_soa *p) {
         c.reordered = false;
         c.reduce_stale = true;
         sync(c);
+        c.least_staging = false;
         p2g_split({&c});
     });
     return EXG_OK;

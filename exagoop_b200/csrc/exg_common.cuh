@@ -127,6 +127,7 @@ struct Params {
     // words between z planes of a node block: B x B, padded where that spreads
     // the W x W columns a warp adds to over more shared-memory banks
     int PS;
+    int nbuf;  // node blocks a P2G thread block works on in turn, 1 or 2
     int gshift;         // log2 of the particles of a fused-G2P work item
     int small;          // fewer than kSmallScene particles in a launch (step_early)
     double gravity[3];

@@ -87,9 +87,13 @@ void launch_dt_finalize(Ctx &c, bool reset);
 void launch_reset_accum(Ctx &c, unsigned long long *bounds, unsigned long long *dtmin);
 void launch_scales_from(Ctx &c, const unsigned long long *bounds);
 void launch_node_reset(Ctx &c);
+// How the P2G splits its work: Params::pshift, nbuf and PS.
+struct P2GSplit {
+    int pshift, nbuf, PS;
+};
 #define EXG_DECL_PREC(sfx)                                                      \
     void launch_state_reduce##sfx(Ctx &c, unsigned long long *bounds, unsigned long long *dtmin); \
-    bool p2g_fits##sfx(const Ctx &c, int ps);                                    \
+    bool p2g_fits##sfx(const Ctx &c, const P2GSplit &s);                         \
     void launch_p2g##sfx(Ctx &c, int flags);                                     \
     void launch_nodes##sfx(Ctx &c, int mode, int flags, bool all_tiles);         \
     void launch_g2p_fused##sfx(Ctx &c, int mode);                                \
@@ -193,6 +197,7 @@ struct Ctx {
     double *stage = nullptr;           // one FP64 particle field: host transfers
     long long stage_cap = 0;
     size_t staging_cap = 0;            // in 64-bit words
+    bool least_staging = false;        // there was no memory for more since the last upload
     size_t staging_max = ~(size_t)0;   // most words it may take (EXG_P2G_STAGING_MAX, in bytes, at creation)
     int nch = 7;
     // control block

@@ -3420,14 +3420,14 @@ struct P2GBatchSrc {
     __device__ __forceinline__ const Ctl *ctl(int s) const { return d[s].ctl; }
     __device__ __forceinline__ void fail(unsigned st) const { atomicOr(&d[0].ctl->status, st); }
 };
-template <class R, int ORD, bool THERM>
-__global__ void __launch_bounds__(P2GVar<R, ORD, 0>::THREADS, 1)
+template <class R, int ORD, bool THERM, int V>
+__global__ void __launch_bounds__(P2GVar<R, ORD, V>::THREADS, 1)
     k_p2g_batch(const SceneDesc<R> *__restrict__ descs, BatchCtl *b, int nv, int pshift) {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ P2GBuf bufs[2];
     const int ns = b->nscenes;
     const P2GBatchSrc<R> src{descs, b, ns, b->pre_active[ns] << pshift, pshift};
-    p2g_run<R, ORD, THERM>(src, smraw, bufs, nv, pshift);
+    p2g_run<R, ORD, THERM, P2GVar<R, ORD, V>::NBUF>(src, smraw, bufs, nv, pshift);
 }
 
 template <class R, bool THERM>
@@ -3683,10 +3683,10 @@ void EXG_SFX(launch_state_reduce)(Ctx &c, unsigned long long *bounds, unsigned l
 }
 
 // Threads and shared memory of a P2G block: as many warps as the shape has,
-// or as their records fit beside the two node blocks.
+// or as their records fit beside the node blocks.
 template <class R, int ORD, bool TH>
-static int p2g_shape(int nv, int threads, size_t &sm) {
-    const size_t fixed = p2g_acc_off() + 2 * p2g_buf_bytes<R>(nv), per = p2g_warp_bytes<R, ORD, TH>();
+static int p2g_shape(int nv, int nbuf, int threads, size_t &sm) {
+    const size_t fixed = p2g_acc_off() + nbuf * p2g_buf_bytes<R>(nv), per = p2g_warp_bytes<R, ORD, TH>();
     const size_t most = 227 * 1024 - sizeof(P2GBuf) * 2 - 64;  // beside the static shared memory
     if (fixed + per > most) throw std::runtime_error("P2G node block does not fit shared memory");
     const int warps = std::min<int>(threads / 32, (int)((most - fixed) / per));
@@ -3694,35 +3694,35 @@ static int p2g_shape(int nv, int threads, size_t &sm) {
     return 32 * warps;
 }
 
-// Whether a block of (nearly) the default shape fits when tiles are split by
-// ps: FP32 cubic whole tiles leave room for 14 of its 16 warps, and the P2G
+// Whether a block of (nearly) the default shape fits with a split: FP32 cubic whole tiles leave room for 14 of its 16 warps, and the P2G
 // and nodal kernels together are no faster with half tiles (876 + 218 us
 // against 884 + 193 us on the 9 M-particle spheres).
 template <class R, int ORD>
-static bool p2g_fits_t(const Ctx &c, int ps) {
+static bool p2g_fits_t(const Ctx &c, const P2GSplit &s) {
     Params P = c.P;
-    P.Bz = (P.T >> ps) + P.hlo + P.hhi;
+    P.PS = s.PS;
+    P.Bz = (P.T >> s.pshift) + P.hlo + P.hhi;
     size_t sm;
     constexpr int nthr = P2GVar<R, ORD, 0>::THREADS;
     try {
-        return c.specs.use_temp ? p2g_shape<R, ORD, true>(p2g_values<true>(P), nthr, sm) * 8 >= nthr * 7
-                                : p2g_shape<R, ORD, false>(p2g_values<false>(P), nthr, sm) * 8 >= nthr * 7;
+        return c.specs.use_temp ? p2g_shape<R, ORD, true>(p2g_values<true>(P), s.nbuf, nthr, sm) * 8 >= nthr * 7
+                                : p2g_shape<R, ORD, false>(p2g_values<false>(P), s.nbuf, nthr, sm) * 8 >= nthr * 7;
     } catch (const std::exception &) {
         return false;
     }
 }
-bool EXG_SFX(p2g_fits)(const Ctx &c, int ps) {
+bool EXG_SFX(p2g_fits)(const Ctx &c, const P2GSplit &s) {
     switch (c.P.uniform_order) {
-        case 1: return p2g_fits_t<EXG_R, 1>(c, ps);
-        case 2: return p2g_fits_t<EXG_R, 2>(c, ps);
-        default: return p2g_fits_t<EXG_R, 3>(c, ps);
+        case 1: return p2g_fits_t<EXG_R, 1>(c, s);
+        case 2: return p2g_fits_t<EXG_R, 2>(c, s);
+        default: return p2g_fits_t<EXG_R, 3>(c, s);
     }
 }
 
 template <class R, int ORD, bool TH, int V>
 static void p2g_v(Ctx &c) {
     size_t sm;
-    const int nthr = p2g_shape<R, ORD, TH>(p2g_values<TH>(c.P), P2GVar<R, ORD, V>::THREADS, sm);
+    const int nthr = p2g_shape<R, ORD, TH>(p2g_values<TH>(c.P), c.P.nbuf, P2GVar<R, ORD, V>::THREADS, sm);
     auto kern = k_p2g<R, ORD, TH, V>;
     EXG_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     const int grid = persistent_grid(kern, sm, nthr);
@@ -3732,7 +3732,8 @@ static void p2g_v(Ctx &c) {
 }
 template <class R, int ORD, bool TH>
 static void p2g_t(Ctx &c) {
-    switch (c.p2g_var) {
+    switch (c.P.nbuf == 1 ? kP2GOneBuf : c.p2g_var) {
+        case kP2GOneBuf: p2g_v<R, ORD, TH, kP2GOneBuf>(c); break;
         case 1: p2g_v<R, ORD, TH, 1>(c); break;
         case 2: p2g_v<R, ORD, TH, 2>(c); break;
         default: p2g_v<R, ORD, TH, 0>(c); break;
@@ -3976,7 +3977,7 @@ static bool batch_descriptors_t(Batch &b) {
     // from the first scene, the nodal kernel each scene's own
     const Params &P0 = b.scenes[0]->P;
     for (const Ctx *c : b.scenes)
-        if (c->P.pshift != P0.pshift || c->P.Bz != P0.Bz || c->P.PS != P0.PS || c->P.T != P0.T)
+        if (c->P.pshift != P0.pshift || c->P.Bz != P0.Bz || c->P.PS != P0.PS || c->P.nbuf != P0.nbuf)
             throw std::runtime_error("internal: the scenes of a batch have different P2G work splits");
     bool changed = false;
     for (int par = 0; par < 2; ++par) {
@@ -4082,19 +4083,23 @@ static void batch_g2p_t(Batch &b, const SceneDesc<R> *d, int B3) {
     EXG_CUDA_OK(cudaGetLastError());
 }
 
-template <class R, int ORD>
-static void batch_p2g_t(Batch &b) {
+template <class R, int ORD, int V>
+static void batch_p2g_v(Batch &b) {
     Ctx &c0 = *b.scenes[0];
     const SceneDesc<R> *d = reinterpret_cast<const SceneDesc<R> *>(b.desc[b.parity]);
     // scenes of a batch share the order, the tile and the split of their tiles
     const int nv = p2g_values<false>(c0.P);
     size_t sm;
-    const int nthr = p2g_shape<R, ORD, false>(nv, P2GVar<R, ORD, 0>::THREADS, sm);
-    auto kern = k_p2g_batch<R, ORD, false>;
+    const int nthr = p2g_shape<R, ORD, false>(nv, c0.P.nbuf, P2GVar<R, ORD, V>::THREADS, sm);
+    auto kern = k_p2g_batch<R, ORD, false, V>;
     EXG_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     const int grid = persistent_grid(kern, sm, nthr);
     kern<<<grid, nthr, sm, b.stream>>>(d, b.bctl, nv, c0.P.pshift);
     EXG_CUDA_OK(cudaGetLastError());
+}
+template <class R, int ORD>
+static void batch_p2g_t(Batch &b) {
+    b.scenes[0]->P.nbuf == 1 ? batch_p2g_v<R, ORD, kP2GOneBuf>(b) : batch_p2g_v<R, ORD, 0>(b);
 }
 template <class R>
 static void batch_nodes_t(Batch &b) {

@@ -43,8 +43,11 @@ constexpr int kP2GChunk = sizeof(R) == 4 ? 32 : 16;
 // (1.1 M spheres).
 constexpr int kP2GVariants = 3;
 static_assert(kP2GVariants == EXG_NUM_VARIANTS, "the launchers dispatch EXG_NUM_VARIANTS P2G variants");
-template <class R, int ORD, int V>
+// The shape with one node block instead of two (Params::nbuf).
+constexpr int kP2GOneBuf = kP2GVariants;
+template <class R, int ORD, int VAR>
 struct P2GVar {
+    static constexpr int NBUF = VAR == kP2GOneBuf ? 1 : 2, V = VAR == kP2GOneBuf ? 0 : VAR;
     static constexpr int TAB[3][3] = {{512, 640, 384}, {640, 512, 384}, {384, 512, 256}};
     static constexpr int THREADS = TAB[sizeof(R) == 8 ? 2 : (P2GStc<ORD>::W == 4 ? 0 : 1)][V];
 };
@@ -388,8 +391,9 @@ __device__ __forceinline__ void p2g_add(const R *rec, int sy, int sz, P2GAcc<R, 
     }
 }
 
-// A block's two node blocks and what its warps know of the item in each.
-// The block works through a sequence of items, item n in buffer n & 1.  Warps
+// A block's node blocks (two; one where the staging of split tiles is too
+// much, see p2g_split) and what its warps know of the item in each.
+// The block works through a sequence of items, item n in buffer n % NBUF.  Warps
 // take rows of an item from `next`; a warp that finds none left leaves for
 // the next item without waiting for the rest.  The last warp to leave writes
 // the item's node block out and zeroes it.  The next item is taken by the
@@ -409,7 +413,7 @@ struct P2GBuf {
     int req, opened, freed;
 };
 
-// Shared memory of a P2G block: spline tables, the two fixed-point node
+// Shared memory of a P2G block: spline tables, the one or two fixed-point node
 // blocks (nv values each, nv a multiple of 4), the warps' records.
 __host__ __device__ constexpr size_t p2g_acc_off() { return (sizeof(SplineTables) + 15) & ~size_t(15); }
 template <class R>
@@ -425,7 +429,7 @@ constexpr int kP2GWaitLimit = 1 << 22;
 // The block's share of a P2G launch.  Src gives the items and, per scene,
 // the grid and the particles: take(scene) is called by one lane and returns
 // the next item or -1.
-template <class R, int ORD, bool THERM, class Src>
+template <class R, int ORD, bool THERM, int NBUF, class Src>
 __device__ __forceinline__ void p2g_run(const Src &src, unsigned char *smraw, P2GBuf *bufs, int nv, int pshift) {
     constexpr int W = P2GStc<ORD>::W, NCH = THERM ? CH_ALL : CH_MOM_END;
     using Lay = P2GRec<R, W, THERM>;
@@ -434,9 +438,9 @@ __device__ __forceinline__ void p2g_run(const Src &src, unsigned char *smraw, P2
     constexpr unsigned FULL = 0xffffffffu;
     SplineTables *tab = reinterpret_cast<SplineTables *>(smraw);
     unsigned char *accs = smraw + p2g_acc_off();
-    R *rec = reinterpret_cast<R *>(accs + 2 * p2g_buf_bytes<R>(nv) + (threadIdx.x >> 5) * p2g_warp_bytes<R, ORD, THERM>());
+    R *rec = reinterpret_cast<R *>(accs + NBUF * p2g_buf_bytes<R>(nv) + (threadIdx.x >> 5) * p2g_warp_bytes<R, ORD, THERM>());
     load_tables(tab);
-    for (int i = threadIdx.x; i < (int)(2 * p2g_buf_bytes<R>(nv) / 16); i += blockDim.x)
+    for (int i = threadIdx.x; i < (int)(NBUF * p2g_buf_bytes<R>(nv) / 16); i += blockDim.x)
         reinterpret_cast<uint4 *>(accs)[i] = make_uint4(0u, 0u, 0u, 0u);
     step_kernel_begin(src.early());
     const int lane = threadIdx.x & 31;
@@ -491,7 +495,7 @@ __device__ __forceinline__ void p2g_run(const Src &src, unsigned char *smraw, P2
     R sc[NO], grav[3];
     int cur = -1;  // scene of sc and grav
     for (int n = 0;; ++n) {
-        const int b = n & 1, s = n >> 1;
+        const int b = n & (NBUF - 1), s = n >> (NBUF - 1);
         P2GBuf &q = bufs[b];
         if (!open(q, s) || !wait(&q.opened, s + 1)) return;
         const int item = *reinterpret_cast<volatile int *>(&q.item);
@@ -519,7 +523,7 @@ __device__ __forceinline__ void p2g_run(const Src &src, unsigned char *smraw, P2
             if (lane == 0) row = atomicAdd(&q.next, 1);
             row = __shfl_sync(FULL, row, 0);
             if (row >= nrow) break;
-            if (row == nrow - 1) {
+            if (NBUF == 2 && row == nrow - 1) {
                 // ahead of the next item's first use, if its buffer is free
                 P2GBuf &qn = bufs[b ^ 1];
                 const int sn = (n + 1) >> 1, f = lane == 0 ? *reinterpret_cast<volatile int *>(&qn.freed) : 0;
@@ -667,5 +671,5 @@ __global__ void __launch_bounds__(P2GVar<R, ORD, V>::THREADS, 1)
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ P2GBuf bufs[2];
     const P2GScene<R> src{P, A, active, start, cell_start, perm, staging, ctl, P.pshift};
-    p2g_run<R, ORD, THERM>(src, smraw, bufs, p2g_values<THERM>(P), P.pshift);
+    p2g_run<R, ORD, THERM, P2GVar<R, ORD, V>::NBUF>(src, smraw, bufs, p2g_values<THERM>(P), P.pshift);
 }

@@ -289,3 +289,58 @@ def test_no_memory_for_the_staging_array(monkeypatch):
     assert np.array_equal(a.pos, b.pos) and np.array_equal(a.rdata, b.rdata)
     ctx.close()
     fresh.close()
+
+
+@pytest.mark.parametrize("precision", [nt.PREC_FP64, nt.PREC_MIXED])
+@pytest.mark.parametrize("case", ["cubic", "quadratic", "thermal"])
+def test_least_staging(case, precision, monkeypatch):
+    # where the staging of split tiles does not fit, tiles stay whole and
+    # their staging is as large as the node blocks themselves: n values of 8
+    # (FP64 12) bytes; every split gives the same bits
+    s, p = lattice_scene(order=2 if case == "quadratic" else 3, thermal=case == "thermal")
+    s.precision = precision
+    s.autotune = 0
+    edge = 8 + (2 if case == "quadratic" else 3)
+    values = -(-(11 if case == "thermal" else 7) * edge ** 3 // 4) * 4
+    tiles = 3 ** 3
+    out = []
+    for limit in (None, tiles * values * (12 if precision == nt.PREC_FP64 else 8)):
+        if limit is not None:
+            monkeypatch.setenv("EXG_P2G_STAGING_MAX", str(limit))
+        ctx = nt.Context(s)
+        ctx.upload(p)
+        ctx.Initialise_Internal_Forces()
+        ctx.step(5)
+        out.append(ctx.download())
+        ctx.P2G_Momentum(1, 1, 1)
+        out.append([ctx.nodes(c) for c in (nt.N_MASS, nt.N_VEL, nt.N_VEL + 1, nt.N_FRC, nt.N_FRC + 2)])
+        ctx.close()
+    assert np.array_equal(out[0].pos, out[2].pos) and np.array_equal(out[0].rdata, out[2].rdata)
+    assert np.array_equal(out[1], out[3])
+
+
+def test_least_staging_in_a_batch(monkeypatch):
+    # a scene without memory for the common split takes the whole batch to the
+    # least one
+    items = [lattice_scene(order=3, seed=k) for k in (1, 2)]
+    items = [(s, elastic(p.pos[:, :n], (1 / 16.,) * 3, 5, speed=0.02)) for (s, p), n in zip(items, (6000, 40))]
+    values = -(-7 * 11 ** 3 // 4) * 4
+    ref = []
+    for s, p in items:
+        ctx = nt.Context(s)
+        ctx.upload(p)
+        ctx.Initialise_Internal_Forces()
+        ctx.step(5)
+        ref.append(ctx.download())
+        ctx.close()
+    monkeypatch.setenv("EXG_P2G_STAGING_MAX", str(27 * values * 12))
+    b = nt.Batch([s for s, _ in items])
+    for sc, (_, p) in zip(b.scenes, items):
+        sc.upload(p)
+        sc.Initialise_Internal_Forces()
+    b.step(2)
+    b.step(3)
+    for sc, r in zip(b.scenes, ref):
+        g = sc.download()
+        assert np.array_equal(g.pos, r.pos) and np.array_equal(g.rdata, r.rdata)
+    b.close()
