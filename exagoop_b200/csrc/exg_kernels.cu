@@ -2568,10 +2568,12 @@ __global__ void k_node_bcs(Params P, Nodes<R> Nd, NodeBCArgs bc, Ctl *ctl) {  //
 
 // The stencil of one particle for the gathers from the dense nodal arrays:
 // its weights (the nearest-node window for uniform quadratic) and, per axis,
-// the node offsets in elements, wrapped on periodic axes.  A node outside the
-// domain has weight 0 and is read at the nearest node of the domain, so the
-// loops over the window have neither tests nor modulo operations.  Weights
-// are formed in FP64 and rounded to R, as the tables' are.
+// the node offsets in elements, wrapped on periodic axes.  The particle may lie
+// outside the domain (on its high face, or moved and not yet redistributed).  A
+// node outside the domain gets weight 0, whatever its spline says, and is read
+// at the nearest node of the domain, so the loops over the window have neither
+// tests nor modulo operations.  Weights are formed in FP64 and rounded to R, as
+// the tables' are.
 template <class R, int ORD>
 struct NodeGather {
     static constexpr int W = ORD == 2 ? 3 : Stc<ORD>::W;
@@ -2608,9 +2610,15 @@ struct NodeGather {
 #pragma unroll
             for (int s = 0; s < W; ++s) {
                 int i = base + s;
-                if (per)
-                    i = i < 0 ? i + nc : (i >= nc ? i - nc : i);
-                i = min(max(i, 0), nc);
+                if (per) {
+                    if (i < 0 || i >= nc) {
+                        i %= nc;
+                        if (i < 0) i += nc;
+                    }
+                } else if (i < 0 || i > nc) {
+                    a[d].w[s] = a[d].dw[s] = R(0);
+                    i = i < 0 ? 0 : nc;
+                }
                 at[d][s] = i * step;
             }
             step *= P.nn[d];
