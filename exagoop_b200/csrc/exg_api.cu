@@ -615,7 +615,7 @@ int status_from_ctl(Ctx &c) {
         return EXG_ERR_OVERFLOW;
     }
     if (st & ST_TIMEOUT) {
-        c.err = "a node-block transfer of the fused G2P did not complete within its wait limit";
+        c.err = "a wait of the P2G or of the fused G2P's node-block transfer ran into its limit";
         return EXG_ERR_TIMEOUT;
     }
     if (st & ST_BOUNDS) {

@@ -3426,16 +3426,16 @@ struct P2GBatchSrc {
     __device__ __forceinline__ const int32_t *perm(int s) const { return d[s].perm; }
     __device__ __forceinline__ long long *staging(int s) const { return d[s].staging; }
     __device__ __forceinline__ const Ctl *ctl(int s) const { return d[s].ctl; }
-    __device__ __forceinline__ void fail(unsigned st) const { atomicOr(&d[0].ctl->status, st); }
+    __device__ __forceinline__ void fail(int s, unsigned st) const { atomicOr(&d[s].ctl->status, st); }
 };
 template <class R, int ORD, bool THERM, int V>
 __global__ void __launch_bounds__(P2GVar<R, ORD, V>::THREADS, 1)
-    k_p2g_batch(const SceneDesc<R> *__restrict__ descs, BatchCtl *b, int nv, int pshift) {
+    k_p2g_batch(const SceneDesc<R> *__restrict__ descs, BatchCtl *b, int nv, int pshift, int rounds) {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ P2GBuf bufs[2];
     const int ns = b->nscenes;
     const P2GBatchSrc<R> src{descs, b, ns, b->pre_active[ns] << pshift, pshift};
-    p2g_run<R, ORD, THERM, P2GVar<R, ORD, V>::NBUF>(src, smraw, bufs, nv, pshift);
+    p2g_run<R, ORD, THERM, P2GVar<R, ORD, V>::NBUF>(src, smraw, bufs, nv, pshift, rounds);
 }
 
 template <class R, bool THERM>
@@ -3735,7 +3735,7 @@ static void p2g_v(Ctx &c) {
     EXG_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     const int grid = persistent_grid(kern, sm, nthr);
     launch_step(c, kern, grid, nthr, sm, c.P, c.A<R>(), c.sb.active, c.sb.tile_start, c.sb.cell_start, c.sb.perm,
-                c.staging, c.ctl);
+                c.staging, c.ctl, p2g_rounds(c.np));
     EXG_CUDA_OK(cudaGetLastError());
 }
 template <class R, int ORD, bool TH>
@@ -4102,7 +4102,9 @@ static void batch_p2g_v(Batch &b) {
     auto kern = k_p2g_batch<R, ORD, false, V>;
     EXG_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     const int grid = persistent_grid(kern, sm, nthr);
-    kern<<<grid, nthr, sm, b.stream>>>(d, b.bctl, nv, c0.P.pshift);
+    long long np = 0;
+    for (const Ctx *c : b.scenes) np += c->np;
+    kern<<<grid, nthr, sm, b.stream>>>(d, b.bctl, nv, c0.P.pshift, p2g_rounds(np));
     EXG_CUDA_OK(cudaGetLastError());
 }
 template <class R, int ORD>

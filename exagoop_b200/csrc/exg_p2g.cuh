@@ -423,14 +423,18 @@ __host__ __device__ constexpr size_t p2g_warp_bytes() {
     return sizeof(R) * P2GRec<R, P2GStc<ORD>::W, THERM>::STRIDE * kP2GChunk<R>;
 }
 // Bounded waits for an item to be opened or written out by another warp of
-// the block (microseconds).
-constexpr int kP2GWaitLimit = 1 << 22;
+// the block, in rounds of kP2GWaitRound polls of 64 ns or more (some tenths of a
+// second).  One warp walks a row whatever it holds (four million FP64 cubic
+// particles in one row take it over a second), so the rounds grow with the
+// particles of the launch: 64 polls a particle, an order more than it takes.
+constexpr int kP2GWaitRound = 1 << 22;
+inline int p2g_rounds(long long np) { return (int)(1 + 64 * np / kP2GWaitRound); }
 
 // The block's share of a P2G launch.  Src gives the items and, per scene,
 // the grid and the particles: take(scene) is called by one lane and returns
 // the next item or -1.
 template <class R, int ORD, bool THERM, int NBUF, class Src>
-__device__ __forceinline__ void p2g_run(const Src &src, unsigned char *smraw, P2GBuf *bufs, int nv, int pshift) {
+__device__ __forceinline__ void p2g_run(const Src &src, unsigned char *smraw, P2GBuf *bufs, int nv, int pshift, int rounds) {
     constexpr int W = P2GStc<ORD>::W, NCH = THERM ? CH_ALL : CH_MOM_END;
     using Lay = P2GRec<R, W, THERM>;
     using Ln = P2GLanes<W>;
@@ -449,16 +453,19 @@ __device__ __forceinline__ void p2g_run(const Src &src, unsigned char *smraw, P2
     int ch0, ch1;
     ln.template first<NCH>(ch0, ch1);
     const bool last = ch0 + (NO - 1) * Ln::STEP < ch1;  // the lane owns its last channel slot
-    auto wait = [&](const int *what, int least) {  // the whole warp; false: gave up
-        for (int it = 0; it < kP2GWaitLimit; ++it) {
-            const int o = lane == 0 ? *reinterpret_cast<const volatile int *>(what) : 0;
-            if (__shfl_sync(FULL, o, 0) >= least) {
-                __threadfence_block();
-                return true;
+    // the whole warp; false: gave up
+    auto wait = [&](const P2GBuf &q, const int *what, int least) {
+#pragma unroll 1
+        for (int r = 0; r < rounds; ++r)
+            for (int it = 0; it < kP2GWaitRound; ++it) {
+                const int o = lane == 0 ? *reinterpret_cast<const volatile int *>(what) : 0;
+                if (__shfl_sync(FULL, o, 0) >= least) {
+                    __threadfence_block();
+                    return true;
+                }
+                __nanosleep(64);
             }
-            __nanosleep(64);
-        }
-        if (lane == 0) src.fail(ST_TIMEOUT);
+        if (lane == 0) src.fail(q.scene, ST_TIMEOUT);
         return false;
     };
     // opens item s of buffer q if no other warp does (the whole warp)
@@ -466,7 +473,7 @@ __device__ __forceinline__ void p2g_run(const Src &src, unsigned char *smraw, P2
         int won = 0;
         if (lane == 0) won = atomicCAS(&q.req, s, s + 1) == s;
         if (!__shfl_sync(FULL, won, 0)) return true;
-        if (!wait(&q.freed, s)) return false;
+        if (!wait(q, &q.freed, s)) return false;
         if (lane == 0) {
             int scene = 0;
             const int item = src.take(scene);
@@ -487,7 +494,10 @@ __device__ __forceinline__ void p2g_run(const Src &src, unsigned char *smraw, P2
         __syncwarp();
         return true;
     };
-    if (threadIdx.x < 2) bufs[threadIdx.x].req = bufs[threadIdx.x].opened = bufs[threadIdx.x].freed = 0;
+    if (threadIdx.x < NBUF) {
+        P2GBuf &q = bufs[threadIdx.x];
+        q.scene = q.req = q.opened = q.freed = 0;
+    }
     __syncthreads();
     P2GAcc<R, THERM> acc[W];
 #pragma unroll
@@ -497,7 +507,7 @@ __device__ __forceinline__ void p2g_run(const Src &src, unsigned char *smraw, P2
     for (int n = 0;; ++n) {
         const int b = n & (NBUF - 1), s = n >> (NBUF - 1);
         P2GBuf &q = bufs[b];
-        if (!open(q, s) || !wait(&q.opened, s + 1)) return;
+        if (!open(q, s) || !wait(q, &q.opened, s + 1)) return;
         const int item = *reinterpret_cast<volatile int *>(&q.item);
         if (item < 0) break;
         const int scene = q.scene;
@@ -661,15 +671,15 @@ struct P2GScene {
     __device__ __forceinline__ const int32_t *perm(int) const { return pm; }
     __device__ __forceinline__ long long *staging(int) const { return stg; }
     __device__ __forceinline__ const Ctl *ctl(int) const { return c; }
-    __device__ __forceinline__ void fail(unsigned st) const { atomicOr(&c->status, st); }
+    __device__ __forceinline__ void fail(int, unsigned st) const { atomicOr(&c->status, st); }
 };
 
 template <class R, int ORD, bool THERM, int V>
 __global__ void __launch_bounds__(P2GVar<R, ORD, V>::THREADS, 1)
     k_p2g(const __grid_constant__ Params P, const __grid_constant__ Parts<R> A, const int *active, const int *start,
-          const int *cell_start, const int32_t *perm, long long *staging, Ctl *ctl) {
+          const int *cell_start, const int32_t *perm, long long *staging, Ctl *ctl, int rounds) {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ P2GBuf bufs[2];
     const P2GScene<R> src{P, A, active, start, cell_start, perm, staging, ctl, P.pshift};
-    p2g_run<R, ORD, THERM, P2GVar<R, ORD, V>::NBUF>(src, smraw, bufs, p2g_values<THERM>(P), P.pshift);
+    p2g_run<R, ORD, THERM, P2GVar<R, ORD, V>::NBUF>(src, smraw, bufs, p2g_values<THERM>(P), P.pshift, rounds);
 }

@@ -65,3 +65,28 @@ def test_p2g_rows(kind, tile, order, precision):
             tol_c = tol
         assert np.abs(a - b).max() <= tol_c * max(np.abs(b).max(), 1e-300), comp
     ctx.close()
+
+
+def test_pile_up_in_one_row():
+    """Four million particles in one cell beside a particle in every tile: the
+    warp that walks the row takes longer than the bound on the other warps'
+    waits for its buffer, which counts only while nothing moves.  The nodal
+    sums are the particles' (an interior cubic stencil sums to 1): relative
+    1e-9, above the rounding of an FP64 sum of four million terms."""
+    n, big = 64, 4_000_000
+    rng = np.random.default_rng(5)
+    cells = np.stack(np.meshgrid(*[np.arange(4, n, 8)] * 3, indexing="ij")).reshape(3, -1)
+    pos = np.concatenate([np.array([[20], [28], [36]]) + rng.uniform(0.01, 0.99, (3, big)), cells + 0.5], axis=1) / n
+    s = scenes.base_specs((0, 0, 0), (1, 1, 1), (n, n, n), 3, nt.PREC_FP64)
+    s.gravity[2] = -9.81
+    s.autotune = 0
+    p = scenes.make_particles(pos, (1.0 / n,) * 3, (2, 2, 2), 1000.0, 0, E=1e3, nu=0.3)
+    p.rdata[nt.R_VEL] = 0.25
+    ctx = nt.Context(s)
+    ctx.upload(p)
+    ctx.P2G_Momentum(1, 1, 1)
+    m, total = ctx.nodes(nt.N_MASS), p.rdata[nt.R_MASS].sum()
+    assert abs(m.sum() / total - 1.0) < 1e-9
+    assert abs((m * ctx.nodes(nt.N_VEL)).sum() / (0.25 * total) - 1.0) < 1e-9
+    assert abs(ctx.nodes(nt.N_FRC + 2).sum() / (-9.81 * total) - 1.0) < 1e-9
+    ctx.close()
