@@ -52,7 +52,11 @@ bool fp64(const Ctx &c) { return c.precision == EXG_PREC_FP64; }
 // eighths.  Fused G2P: the same scene 159 / 105 / 67 / 43 / 35 us with items of
 // 4096 / 2048 / 1024 / 512 / 256 particles, 540 thousand cubic particles 154 /
 // 159 / 115 / 109 / 117 us.  An item whose node block comes by plain loads
-// (periodic grids) costs more: 0.9 M particles 139 / 150 / 154 / 155 / 182 us.
+// (periodic grids) costs more, as its particles wait for it: us a step with at
+// least 148 / 300 / 600 / 1000 / 2000 items 98 / 102 / 102 / 102 / 102 at 124
+// thousand particles, 176 / 181 / 173 / 183 / 184 at 0.4 M, 297 / 304 / 310 / 312
+// / 341 at 1 M (FP64 533 / 540 / 547 / 533 / 556), 557 / 559 / 563 / 564 / 590 at
+// 2 M.
 constexpr long long kP2GItems = 148 * 3, kG2PItems = 1000, kG2PItemsPlain = 148;
 
 template <class T>
@@ -408,7 +412,7 @@ void p2g_split(const std::vector<Ctx *> &scenes) {
             for (Ctx *x : scenes) x->least_staging = true;
         }
     }
-    const int small = n < kSmallScene;
+    const int small = n <= kSmallScene && !c.specs.use_temp;
     for (Ctx *x : scenes) {
         Params &P = x->P;
         int gs = kG2PMaxShift;

@@ -70,7 +70,9 @@ struct Ctl {
 // 8^3 tile) stay whole: items of 1024 made the 9 M-particle sphere step's G2P
 // 5 % slower (FP64, whose node block arrives single-buffered, 15 %).
 constexpr int kG2PMaxShift = 12, kG2PMinShift = 8;
-constexpr long long kSmallScene = 1 << 16;
+// Up to here, without temperature, a launch is a small scene's (step_early has
+// the figures).
+constexpr long long kSmallScene = 1 << 14;
 
 // Per-tile stride of the P2G staging array, in 64-bit words, for nv
 // fixed-point values: FP32 state one 64-bit integer per value; FP64 state
@@ -129,7 +131,7 @@ struct Params {
     int PS;
     int nbuf;  // node blocks a P2G thread block works on in turn, 1 or 2
     int gshift;         // log2 of the particles of a fused-G2P work item
-    int small;          // fewer than kSmallScene particles in a launch (step_early)
+    int small;          // at most kSmallScene particles in a launch, no temperature (step_early)
     double gravity[3];
     int external_loads;
     double slab_lo[3], slab_hi[3], extforce[3];

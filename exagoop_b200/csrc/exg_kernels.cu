@@ -87,9 +87,13 @@ __device__ __forceinline__ void step_kernel_begin(bool early = true) {
     if (early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 // The P2G, nodal and fused G2P kernels let the next kernel in early only in
-// small scenes: waiting blocks take shared memory and L1 from the one that runs
-// (early starts there: 8 thousand particles 63 -> 56 us a step, 15 thousand 89
-// -> 86, but a 290 thousand-particle MUSL step 571 -> 608).
+// small scenes: waiting blocks take shared memory and L1 from the one that runs.
+// us a step without / with early starts there: FP64 linear 8 thousand particles
+// 56.9 / 55.5, 16 thousand 57.6 / 56.1; quadratic dam break 15 thousand FP64
+// 84.0 / 83.0, mixed 64.3 / 63.4, 25 thousand FP64 84.8 / 89.0, mixed 65.3 /
+// 65.3, 124 thousand FP64 156 / 162; cubic spheres 18 thousand mixed 66.8 / 66.9,
+// FP64 90.8 / 93.4. With temperature slower at every size: 12 thousand FP64 120 /
+// 130, MUSL 210 / 251, 43 thousand 152 / 180, MUSL 267 / 321.
 __device__ __forceinline__ bool step_early(const Params &P) { return P.small; }
 
 __device__ __forceinline__ void load_tables(SplineTables *dst) {
@@ -3575,8 +3579,9 @@ static int persistent_grid(K kern, size_t smem, int threads = kThreads) {
 // Launch of a step kernel (one that passes step_kernel_begin): its blocks may
 // start while the kernel before it in the stream drains, which takes a few
 // microseconds of launch latency off each of a step's kernels.  Not in large
-// scenes, where that is nothing and the waiting blocks disturb (9 M particles
-// 2394 -> 2430 us a step, the sort and the P2G slower).
+// scenes, where that is nothing and the waiting blocks disturb.  us a step
+// without / with: 0.5 M particles 253 / 249, 1.1 M 411 / 407, 1.6 M with heat 751 /
+// 754, 2.0 M 527 / 529, 2.2 M 698 / 698, 4.3 M 1256 / 1265, 9 M 2398 / 2415.
 constexpr long long kEarlyLaunch = 1 << 21;
 template <class... E, class... A>
 static void launch_step(const Ctx &c, void (*kern)(E...), int grid, int threads, size_t smem, A &&...args) {
@@ -3645,10 +3650,14 @@ void launch_sort_rest(Ctx &c, bool touched_list, const unsigned long long *bound
     size_t sm = sizeof(int) * (3 * ncell + kSortCap);
     EXG_CUDA_OK(cudaFuncSetAttribute(k_tile_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     // A tile's sort is a chain of passes over its particles, so while there are
-    // fewer tiles than blocks at a time a tile gets a block of 1024 threads (15
-    // thousand particles 28 -> 11 us, 1.1 M 34 -> 23 us); otherwise 256, of
-    // which more fit an SM.
-    const bool few = c.np < 148ll * 8 * 512 * 2;
+    // fewer tiles than blocks at a time a tile of edge 8 gets a block of 1024
+    // threads (15 thousand particles 28 -> 11 us, 1.1 M 34 -> 23 us); otherwise
+    // 256, of which more fit an SM. us a step with 256 / 1024 threads: 124
+    // thousand 116 / 97, 1.0 M 321 / 306, 2.2 M 699 / 696, 3.7 M 883 / 885. A tile
+    // of edge 4 has too few particles for 1024 threads (416 thousand 177 / 185,
+    // 1.1 M 457 / 473); one particle a cell is not told apart (0.5 M 619 / 624,
+    // 1.0 M 711 / 722).
+    const bool few = c.P.T == 8 && c.np < 148ll * 8 * 512 * 2;
     const int thr = few ? 1024 : kThreads;
     const int sgrid = persistent_grid(k_tile_sort, sm, thr);
     // no more blocks than the scene has tiles (small scenes of a batch)
