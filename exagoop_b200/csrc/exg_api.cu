@@ -1535,7 +1535,7 @@ void autotune_impl(Ctx &c) {
         for (int v = 0; v < EXG_NUM_VARIANTS; ++v) {
             c.p2g_var = v;
             c.tune_ms[0][v] = time_launches(c, 3, [&] {
-                launch_scales_from(c, c.bounds2);  // also resets the P2G tile counter
+                launch_scales_from(c, c.bounds2);  // also resets the P2G item counter
                 DISPATCH(launch_p2g, c, flags);
             });
         }

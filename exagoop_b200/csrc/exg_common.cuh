@@ -57,15 +57,15 @@ struct Ctl {
     int n_touched_tiles;
     long long n_sorted;                // particles inside the domain after the sort
     unsigned long long lost_fill;      // next slot for out-of-domain particles in the re-ordered storage
-    int next_p2g;                      // dynamic tile counter of the P2G kernel (reset with the fixed-point scales)
+    int next_p2g;                      // dynamic item counter of the P2G kernel (reset with the fixed-point scales)
     int next_g2p;                      // dynamic item counter of the fused G2P (reset by k_nodes)
     int n_g2p_items;                   // work items of the fused G2P
     int pad2;
 };
 // Particles of one work item of the fused G2P, as a power of two (the host
-// chooses it per particle count, g2p_chunk).  A tile of more particles (a
+// chooses it per particle count, p2g_split).  A tile of more particles (a
 // pile-up) is split into several items, so that no item is much longer than
-// an ordinary tile.  Each item stages its tile's node block again, so where
+// an ordinary tile.  (The batched G2P takes whole tiles.)  Each item stages its tile's node block again, so where
 // there are tiles enough for the GPU ordinary ones (8 particles per cell of an
 // 8^3 tile) stay whole: items of 1024 made the 9 M-particle sphere step's G2P
 // 5 % slower (FP64, whose node block arrives single-buffered, 15 %).
@@ -82,8 +82,9 @@ EXG_HD constexpr long long stg_stride(long long nv) { return sizeof(R) == 4 ? nv
 
 // Control block of a batch of independent scenes advanced by one launch per
 // kernel: prefix sums of the scenes' tile counts and the batch's dynamic
-// tile counters (k_batch_plan fills them before each step's batched
-// kernels).
+// item counters (k_batch_plan fills them before each step's batched
+// kernels): P2G items are 1 << pshift to a tile, the nodal kernel, the G2P and
+// the sort take whole tiles.
 constexpr int kMaxScenes = 1024;
 struct BatchCtl {
     int nscenes;
@@ -210,8 +211,8 @@ struct Nodes {
     // interleaved copy of the fields the fused G2P reads, written by the
     // nodal kernel of a fused step: per node v(3), dv(3) (FP32 padded to 8
     // words, FP64 6), so one 4-D TMA box fetches a tile's whole node block in
-    // the layout the G2P uses; null when the G2P stages nodes itself
-    // (periodic axes)
+    // the layout the G2P uses; the plain staging (periodic axes, batches)
+    // reads it too, so every context has it
     R *rec;
 };
 template <class R>

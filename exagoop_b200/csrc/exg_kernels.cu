@@ -502,8 +502,8 @@ __device__ __forceinline__ void tile_sort_item(int *sm, const int *active, const
         for (int r = b; r < e; ++r) rank += (ent[r] < i);
         perm[s0 + b + rank] = i;
     }
-    // cell ranges of this tile (relative to the tile start), for the
-    // per-cell P2G
+    // cell ranges of this tile (relative to the tile start), for the P2G's
+    // rows
     int *cs = cell_start + (long long)w * (ncell + 1);
     for (int c = threadIdx.x; c < ncell; c += blockDim.x) cs[c] = cst[c];
     if (threadIdx.x == 0) {
@@ -717,13 +717,14 @@ __global__ void k_reset_accum(unsigned long long *bounds, unsigned long long *dt
 
 // ---------------------------------------------------------------- K2 P2G
 // deposit_onto_grid_momentum (mpm_particle_grid_ops.cpp:405-588) and the
-// thermal deposit (:703-844), one CTA per non-empty tile.  Contributions are
-// converted to 64-bit fixed point with a per-channel power-of-two scale and
-// accumulated with integer shared-memory atomics: integer addition is
-// associative, so node sums do not depend on thread scheduling and the
-// result is identical run to run.  The CTA then stores its whole node block
-// (tile plus halo) as one partial; the nodal kernel adds the <= 8 partials
-// covering each node.
+// thermal deposit (:703-844), one work item per non-empty tile or slab of z
+// planes of one.  Contributions are converted to fixed point (FP32 64 bits, FP64
+// 96) with a per-channel power-of-two scale and accumulated with integer
+// shared-memory atomics: integer addition is associative, so node sums do not
+// depend on thread scheduling and the result is identical run to run.  An item's
+// node block (its cells plus halo) is stored whole as one partial; the nodal
+// kernel adds the partials covering each node: those of up to 8 tiles, and of
+// each tile's slabs that reach the node's plane.
 template <int ORD>
 struct Stc {
     static constexpr int W = (ORD == 1) ? 2 : 4;
@@ -742,8 +743,8 @@ __device__ __forceinline__ T sel(const T (&a)[W], int i) {
 // ---------------------------------------------------------------- K2 helpers
 // A node's fixed-point sum in shared memory.
 // FP32 state (scale bound 2^55, kFxBits32): two 32-bit words; without
-// carries, lo collects the low 24 bits of each addend (at most 64 addends
-// per node and tile, so lo < 2^30) and hi the arithmetic upper part, which
+// carries, lo collects the low 24 bits of each addend (one for each of the at
+// most W x W = 16 rows that reach a node, so lo < 2^28) and hi the arithmetic upper part, which
 // fits 32 bits; the value is hi * 2^24 + lo and both adds are
 // fire-and-forget reductions.
 // FP64 state (bound 2^93, kFxBits64): a 64-bit low word and a 32-bit high
@@ -846,7 +847,7 @@ struct FxSum<double> {
     }
 };
 
-// Stencil width of the per-cell P2G: cells (linear, cubic, mixed orders) or
+// Stencil width of the P2G: cells (linear, cubic, mixed orders) or
 // nearest-node bins (uniform quadratic).  The block index of stencil slot s
 // is (local cell or bin) + s in every case.
 template <int ORD>
@@ -2047,9 +2048,9 @@ __device__ __forceinline__ bool all_finite(const R *a, int n) {
     return ok;
 }
 
-// Fused K4: one CTA per non-empty tile.  The tile's node block (velocity
-// and delta-velocity, halo included) is staged in shared memory once; each
-// particle of the tile is gathered from storage A through the sort
+// Fused K4: one block per work item, a non-empty tile or 1 << gshift of its
+// particles.  The tile's node block (velocity and delta-velocity, halo
+// included) is staged in shared memory once; each particle of the item is gathered from storage A through the sort
 // permutation and written to storage B at its sorted position, so the
 // particle arrays are physically re-ordered by cell every step at no extra
 // pass.  GM_VEL updates velocity in place in A instead.
@@ -3266,7 +3267,7 @@ __device__ __forceinline__ int scene_of(const int *pre, int ns, int i) {
 }
 
 // Prefix sums of the scenes' active and touched tile counts; resets the
-// batch's tile counters.  One block.
+// batch's item counters.  One block.
 __global__ void k_batch_plan(BatchCtl *b, Ctl *const *ctls) {
     __shared__ int sh[34];
     __shared__ int ca, ct;
