@@ -38,8 +38,8 @@ constexpr int kP2GChunk = sizeof(R) == 4 ? 32 : 16;
 // Launch shapes: most threads per block (fewer where their records do not
 // fit shared memory).  The kernel waits on fixed latencies, shared memory and
 // its particle loads, so warps decide its speed until registers spill: FP32
-// cubic 993 / 876 / 915 us at 12 / 16 / 20 warps (9 M spheres), quadratic
-// 787 / 689 / 623 us (8 M dam break); FP64 cubic 315 / 430 us at 12 / 16
+// cubic 988 / 852 / 925 us at 12 / 16 / 20 warps (9 M spheres), quadratic
+// 800 / 699 / 622 us (8 M dam break); FP64 cubic 315 / 430 us at 12 / 16
 // (1.1 M spheres).
 constexpr int kP2GVariants = 3;
 static_assert(kP2GVariants == EXG_NUM_VARIANTS, "the launchers dispatch EXG_NUM_VARIANTS P2G variants");
