@@ -3435,12 +3435,12 @@ struct P2GBatchSrc {
 };
 template <class R, int ORD, bool THERM, int V>
 __global__ void __launch_bounds__(P2GVar<R, ORD, V>::THREADS, 1)
-    k_p2g_batch(const SceneDesc<R> *__restrict__ descs, BatchCtl *b, int nv, int pshift, int rounds) {
+    k_p2g_batch(const SceneDesc<R> *__restrict__ descs, BatchCtl *b, int nv, int pshift) {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ P2GBuf bufs[2];
     const int ns = b->nscenes;
     const P2GBatchSrc<R> src{descs, b, ns, b->pre_active[ns] << pshift, pshift};
-    p2g_run<R, ORD, THERM, P2GVar<R, ORD, V>::NBUF>(src, smraw, bufs, nv, pshift, rounds);
+    p2g_run<R, ORD, THERM, P2GVar<R, ORD, V>::NBUF>(src, smraw, bufs, nv, pshift);
 }
 
 template <class R, bool THERM>
@@ -3745,7 +3745,7 @@ static void p2g_v(Ctx &c) {
     EXG_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     const int grid = persistent_grid(kern, sm, nthr);
     launch_step(c, kern, grid, nthr, sm, c.P, c.A<R>(), c.sb.active, c.sb.tile_start, c.sb.cell_start, c.sb.perm,
-                c.staging, c.ctl, p2g_rounds(c.np));
+                c.staging, c.ctl);
     EXG_CUDA_OK(cudaGetLastError());
 }
 template <class R, int ORD, bool TH>
@@ -4112,9 +4112,7 @@ static void batch_p2g_v(Batch &b) {
     auto kern = k_p2g_batch<R, ORD, false, V>;
     EXG_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     const int grid = persistent_grid(kern, sm, nthr);
-    long long np = 0;
-    for (const Ctx *c : b.scenes) np += c->np;
-    kern<<<grid, nthr, sm, b.stream>>>(d, b.bctl, nv, c0.P.pshift, p2g_rounds(np));
+    kern<<<grid, nthr, sm, b.stream>>>(d, b.bctl, nv, c0.P.pshift);
     EXG_CUDA_OK(cudaGetLastError());
 }
 template <class R, int ORD>

@@ -423,18 +423,18 @@ __host__ __device__ constexpr size_t p2g_warp_bytes() {
     return sizeof(R) * P2GRec<R, P2GStc<ORD>::W, THERM>::STRIDE * kP2GChunk<R>;
 }
 // Bounded waits for an item to be opened or written out by another warp of
-// the block, in rounds of kP2GWaitRound polls of 64 ns or more (some tenths of a
-// second).  One warp walks a row whatever it holds (four million FP64 cubic
-// particles in one row take it over a second), so the rounds grow with the
-// particles of the launch: 64 polls a particle, an order more than it takes.
-constexpr int kP2GWaitRound = 1 << 22;
-inline int p2g_rounds(long long np) { return (int)(1 + 64 * np / kP2GWaitRound); }
+// the block, in polls of 64 ns or more: a minute at least.  One warp walks a row
+// whatever it holds (four million FP64 cubic particles in one row take it over
+// a second), and as many as fit the device's memory take it less than that.  A
+// bound by the particles of the launch cost the quadratic P2G 1.6 % (0.9 M
+// particles 106.5 -> 108.2 us), a constant one nothing.
+constexpr int kP2GWaitLimit = 1 << 30;
 
 // The block's share of a P2G launch.  Src gives the items and, per scene,
 // the grid and the particles: take(scene) is called by one lane and returns
 // the next item or -1.
 template <class R, int ORD, bool THERM, int NBUF, class Src>
-__device__ __forceinline__ void p2g_run(const Src &src, unsigned char *smraw, P2GBuf *bufs, int nv, int pshift, int rounds) {
+__device__ __forceinline__ void p2g_run(const Src &src, unsigned char *smraw, P2GBuf *bufs, int nv, int pshift) {
     constexpr int W = P2GStc<ORD>::W, NCH = THERM ? CH_ALL : CH_MOM_END;
     using Lay = P2GRec<R, W, THERM>;
     using Ln = P2GLanes<W>;
@@ -455,16 +455,14 @@ __device__ __forceinline__ void p2g_run(const Src &src, unsigned char *smraw, P2
     const bool last = ch0 + (NO - 1) * Ln::STEP < ch1;  // the lane owns its last channel slot
     // the whole warp; false: gave up
     auto wait = [&](const P2GBuf &q, const int *what, int least) {
-#pragma unroll 1
-        for (int r = 0; r < rounds; ++r)
-            for (int it = 0; it < kP2GWaitRound; ++it) {
-                const int o = lane == 0 ? *reinterpret_cast<const volatile int *>(what) : 0;
-                if (__shfl_sync(FULL, o, 0) >= least) {
-                    __threadfence_block();
-                    return true;
-                }
-                __nanosleep(64);
+        for (int it = 0; it < kP2GWaitLimit; ++it) {
+            const int o = lane == 0 ? *reinterpret_cast<const volatile int *>(what) : 0;
+            if (__shfl_sync(FULL, o, 0) >= least) {
+                __threadfence_block();
+                return true;
             }
+            __nanosleep(64);
+        }
         if (lane == 0) src.fail(q.scene, ST_TIMEOUT);
         return false;
     };
@@ -494,10 +492,8 @@ __device__ __forceinline__ void p2g_run(const Src &src, unsigned char *smraw, P2
         __syncwarp();
         return true;
     };
-    if (threadIdx.x < NBUF) {
-        P2GBuf &q = bufs[threadIdx.x];
-        q.scene = q.req = q.opened = q.freed = 0;
-    }
+    if (threadIdx.x < 2)
+        bufs[threadIdx.x].scene = bufs[threadIdx.x].req = bufs[threadIdx.x].opened = bufs[threadIdx.x].freed = 0;
     __syncthreads();
     P2GAcc<R, THERM> acc[W];
 #pragma unroll
@@ -677,9 +673,9 @@ struct P2GScene {
 template <class R, int ORD, bool THERM, int V>
 __global__ void __launch_bounds__(P2GVar<R, ORD, V>::THREADS, 1)
     k_p2g(const __grid_constant__ Params P, const __grid_constant__ Parts<R> A, const int *active, const int *start,
-          const int *cell_start, const int32_t *perm, long long *staging, Ctl *ctl, int rounds) {
+          const int *cell_start, const int32_t *perm, long long *staging, Ctl *ctl) {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ P2GBuf bufs[2];
     const P2GScene<R> src{P, A, active, start, cell_start, perm, staging, ctl, P.pshift};
-    p2g_run<R, ORD, THERM, P2GVar<R, ORD, V>::NBUF>(src, smraw, bufs, p2g_values<THERM>(P), P.pshift, rounds);
+    p2g_run<R, ORD, THERM, P2GVar<R, ORD, V>::NBUF>(src, smraw, bufs, p2g_values<THERM>(P), P.pshift);
 }
