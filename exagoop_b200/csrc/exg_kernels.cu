@@ -2591,6 +2591,13 @@ struct NodeGather {
             const int nc = P.nc[d];
             const bool per = P.periodic[d];
             int base;
+            // a node outside the domain gets no weight (the quadratic weights have that)
+            auto inside = [&] {
+                if (per) return;
+#pragma unroll
+                for (int s = 0; s < W; ++s)
+                    if (base + s < 0 || base + s > nc) a[d].w[s] = a[d].dw[s] = R(0);
+            };
             if constexpr (ORD == 2 || ORD == 3) {
                 const int c = ORD == 2 ? dual_bin(P, d, x[d]) : iv[d];
                 const double xw = ORD == 2 ? dual_x(P, d, x[d]) : x[d];
@@ -2607,24 +2614,23 @@ struct NodeGather {
                     dual_axis_weights<R>(tab, P, d, xw, c, false, a[d]);
                 } else {
                     axis_weights<R, W, -1>(tab, P, d, xw, c, a[d]);
+                    inside();
                 }
             } else {
                 axis_weights<R, W, Stc<ORD>::LO>(tab, P, d, x[d], iv[d], a[d]);
                 base = iv[d] + Stc<ORD>::LO;
+                inside();
+            }
+            if (per && (base < 0 || base >= nc)) {  // periods away: to [0, nc)
+                base %= nc;
+                if (base < 0) base += nc;
             }
 #pragma unroll
             for (int s = 0; s < W; ++s) {
                 int i = base + s;
-                if (per) {
-                    if (i < 0 || i >= nc) {
-                        i %= nc;
-                        if (i < 0) i += nc;
-                    }
-                } else if (i < 0 || i > nc) {
-                    a[d].w[s] = a[d].dw[s] = R(0);
-                    i = i < 0 ? 0 : nc;
-                }
-                at[d][s] = i * step;
+                if (per)
+                    i = i >= nc ? i - nc : i;
+                at[d][s] = min(max(i, 0), nc) * step;
             }
             step *= P.nn[d];
         }
@@ -2637,7 +2643,7 @@ struct NodeGather {
 // index and a copy of the parameters per node) the gather of 140 thousand
 // cubic particles took 489 us, 31 us now.
 template <class R, int ORD>
-__global__ void __launch_bounds__(kThreads) k_g2p_simple(const __grid_constant__ Params P, Parts<R> A, Nodes<R> Nd,
+__global__ void __launch_bounds__(kThreads, ORD == 1 ? 2 : 0) k_g2p_simple(const __grid_constant__ Params P, Parts<R> A, Nodes<R> Nd,
                                                          long long np, int upd_vel, int upd_sr, double dt) {
     __shared__ SplineTables tab;
     load_tables(&tab);
