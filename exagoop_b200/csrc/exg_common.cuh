@@ -122,6 +122,7 @@ struct Params {
     int T;              // tile edge (cells, or nearest-node bins when dual)
     int tshift;         // log2(T)
     int ntile[3];
+    int nbuf;           // node blocks a P2G thread block works on in turn, 1 or 2
     long long ntiles;
     int hlo, hhi, B;    // node-block halo below/above and edge B = T+hlo+hhi
     // P2G work items per tile, 1 << pshift: each takes T >> pshift z planes of
@@ -130,7 +131,6 @@ struct Params {
     // words between z planes of a node block: B x B, padded where that spreads
     // the W x W columns a warp adds to over more shared-memory banks
     int PS;
-    int nbuf;  // node blocks a P2G thread block works on in turn, 1 or 2
     int gshift;         // log2 of the particles of a fused-G2P work item
     int small;          // at most kSmallScene particles in a launch, no temperature (step_early)
     double gravity[3];
